@@ -34,6 +34,8 @@ struct LbmPlan {
     unsigned* status;      // device status word (lbm_plan_status), inside the reduction scratch
     uint32_t* rowmask;     // row summary of the flag field last finalized with this plan
     mutable const uint8_t* rowmask_flags;  // that flag field (sweeps given it use the summary)
+    mutable uint32_t* walls;               // wall words of that flag field (three planes), or nullptr
+    mutable bool walls_valid;              // they belong to rowmask_flags
     void* ubb_rho;         // compressible + moving UBB walls: density gathered before the sweep
     const int* ubb_block;  // per-link boundary tables (lbm_plan_set_links), caller-owned
     const double* ubb_link_vel;
@@ -123,6 +125,8 @@ Grid make_grid(const LbmPlan* p, const int64_t s[4], const uint8_t* flags) {
     g.fsy = g.nx + 2;
     g.fsz = (g.nx + 2) * (g.ny + 2);
     g.rowmask = nullptr;
+    g.walls = nullptr;
+    g.wall_plane = unsigned(g.nx) * unsigned(g.ny) * unsigned(g.nz);
     return g;
 }
 
@@ -474,6 +478,57 @@ __global__ void k_flags_finalize(Grid g) {
     fl[fc] = (uint8_t)v;
 }
 
+// Wall words of a finalized flag field (WALL_* in lbm_common.cuh): three planes of one word per
+// interior cell.
+template <int Q>
+__global__ void __launch_bounds__(256) k_wall_words(Grid g, uint32_t* words) {
+    using L = Lat<Q>;
+    const int x = blockIdx.x * blockDim.x + threadIdx.x;
+    const int y = blockIdx.y * blockDim.y + threadIdx.y;
+    const int z = blockIdx.z;
+    if (x >= g.nx || y >= g.ny) return;
+    const uint8_t* cell = g.flags + ((x + 1) + (y + 1) * g.fsy + (z + 1) * g.fsz);
+    const int fl = *cell;
+    uint32_t w = 0, ubb = 0, per_link = 0;
+    if (fl & FLAG_TYPE_MASK) {
+        w = WALL_SELF;
+    } else if (fl & FLAG_NEAR_WALL) {
+        NbrOffsets fo;
+        Grid gf = g;
+        gf.sy = g.fsy;
+        gf.sz = g.fsz;
+        fo.init(gf, x, y, z);
+        unsigned types = 0;   // bit t: a link to a cell of type t
+#pragma unroll
+        for (int i = 1; i < Q; ++i) {
+            const int t = cell[fo.off(-L::cx(i), -L::cy(i), -L::cz(i))] & FLAG_TYPE_MASK;
+            types |= 1u << t;
+            if (t == FLAG_NOSLIP || flag_is_ubb(t)) w |= 1u << i;
+            if (flag_is_ubb(t)) ubb |= 1u << i;
+            if (t >= FLAG_FREE_SLIP) per_link |= 1u << i;
+        }
+        if (types & ((1u << FLAG_FIXED_DENSITY) | (1u << FLAG_FIXED_DENSITY1))) w |= WALL_FIXED_DENSITY;
+        if (per_link) w |= WALL_PER_LINK;
+        if (ubb) {
+            w |= WALL_UBB;
+            const unsigned numbers = (types >> FLAG_UBB0) & ((1u << MAX_UBB) - 1u);
+            ubb |= (numbers & (numbers - 1u)) ? WALL_UBB_MIXED : uint32_t(__ffs(int(numbers)) - 1) << WALL_UBB_SHIFT;
+        }
+    }
+    const size_t c = size_t(x) + size_t(g.nx) * (size_t(y) + size_t(g.ny) * z);
+    words[c] = w;
+    words[c + g.wall_plane] = ubb;
+    words[c + 2 * size_t(g.wall_plane)] = per_link;
+}
+
+cudaError_t launch_wall_words(int q, const Grid& g, uint32_t* words, cudaStream_t s) {
+    dim3 grid, block;
+    launch_shape(g, 1, grid, block);
+    if (q == 19) k_wall_words<19><<<grid, block, 0, s>>>(g, words);
+    else k_wall_words<27><<<grid, block, 0, s>>>(g, words);
+    return cudaGetLastError();
+}
+
 // Optimal third-order rates w3..w5 (before the per-cell limiters) and the parameters a, b of the
 // fourth-order correction for shear rate w1 and bulk rate w2 (Geier et al. 2017, eq. 111-116;
 // methods/cumulantbased/fourth_order_correction.py:79-97, :149-170).  False if a denominator vanishes.
@@ -693,6 +748,8 @@ int lbm_plan_create(const LbmPlanDesc* desc, LbmPlan** out) {
     p->ubb_rho = nullptr;
     p->rowmask = nullptr;
     p->rowmask_flags = nullptr;
+    p->walls = nullptr;
+    p->walls_valid = false;
     if (sweep_launcher(p, PAT_PULL) == nullptr) {
         cudaFree(p->partial);
         delete p;
@@ -733,6 +790,7 @@ int lbm_plan_destroy(LbmPlan* p) {
     if (p->partial) cudaFree(p->partial);
     if (p->ubb_rho) cudaFree(p->ubb_rho);
     if (p->rowmask) cudaFree(p->rowmask);
+    if (p->walls) cudaFree(p->walls);
     delete p;
     return LBM_OK;
 }
@@ -787,7 +845,10 @@ static int launch_sweep_checked(const LbmPlan* p, const void* src, void* dst, co
     a.ubb_link_vel = p->ubb_link_vel;
     a.link_code = p->link_code;
     a.link_value = p->link_value;
-    if (flags != nullptr && flags == p->rowmask_flags) a.g.rowmask = p->rowmask;
+    if (flags != nullptr && flags == p->rowmask_flags) {
+        a.g.rowmask = p->rowmask;
+        if (p->walls_valid) a.g.walls = p->walls;
+    }
     if (flags != nullptr && p->ubb_rho != nullptr && needs_ubb_density(&p->desc, p->ubb_link_mask)) {
         UbbLauncher U = p->q == 19 ? ubb_launcher_q<19>(p->store, pat) : ubb_launcher_q<27>(p->store, pat);
         if (U == nullptr) return fail(LBM_E_UNSUPPORTED, "no wall-density kernel for this storage type / pattern");
@@ -999,12 +1060,27 @@ int lbm_flags_finalize(const LbmPlan* p, uint8_t* flags, void* stream) {
     if (e != cudaSuccess) return cuda_fail(e, "flag finalize launch");
     // the row summary the sweeps of this plan use with this flag field
     p->rowmask_flags = nullptr;
+    p->walls_valid = false;
     e = cudaMemsetAsync(p->rowmask, 0, rowmask_bytes(p), st);
     if (e != cudaSuccess) return cuda_fail(e, "clearing the row summary");
     const int rows = g.ny * g.nz;
     k_row_mask<<<(rows + 255) / 256, 256, 0, st>>>(g, p->rowmask);
     e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(e, "row summary launch");
+    // and their wall words; without the memory for them (or while a graph is being captured, when it
+    // cannot be allocated) the sweeps take the walls from the flags
+    if (p->walls == nullptr) {
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(st, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone &&
+            cudaMalloc(&p->walls, 3 * sizeof(uint32_t) * size_t(g.wall_plane)) != cudaSuccess)
+            p->walls = nullptr;
+        cudaGetLastError();
+    }
+    if (p->walls != nullptr) {
+        e = launch_wall_words(p->q, g, p->walls, st);
+        if (e != cudaSuccess) return cuda_fail(e, "wall word launch");
+        p->walls_valid = true;
+    }
     p->rowmask_flags = flags;
     return LBM_OK;
 }
@@ -1196,6 +1272,7 @@ struct LbmBatch {
     LbmBatchTiling tiling;
     int64_t n_tiles, grid_blocks, cells;
     SweepArgs* d_domains;      // [2][n_domains]: parity 0 and parity 1 source/destination
+    uint32_t* d_walls;         // wall words of every domain with flags
     BatchTile* d_tiles;
 };
 
@@ -1367,7 +1444,18 @@ int lbm_batch_create(const LbmPlanDesc* common, const LbmDomainDesc* domains, in
     b->cells = cells;
     b->d_domains = nullptr;
     b->d_tiles = nullptr;
-    e = cudaMalloc(&b->d_domains, sizeof(SweepArgs) * args.size());
+    b->d_walls = nullptr;
+    size_t wall_words = 0;
+    for (int k = 0; k < n_domains; ++k)
+        if (domains[k].flags_offset >= 0) wall_words += 3 * size_t(args[k].g.wall_plane);
+    if (wall_words > 0) e = cudaMalloc(&b->d_walls, sizeof(uint32_t) * wall_words);
+    wall_words = 0;
+    for (int k = 0; k < n_domains && e == cudaSuccess; ++k) {
+        if (domains[k].flags_offset < 0) continue;
+        args[k].g.walls = args[n_domains + k].g.walls = b->d_walls + wall_words;
+        wall_words += 3 * size_t(args[k].g.wall_plane);
+    }
+    if (e == cudaSuccess) e = cudaMalloc(&b->d_domains, sizeof(SweepArgs) * args.size());
     if (e == cudaSuccess) e = cudaMalloc(&b->d_tiles, sizeof(BatchTile) * tiles.size());
     if (e == cudaSuccess)
         e = cudaMemcpy(b->d_domains, args.data(), sizeof(SweepArgs) * args.size(), cudaMemcpyHostToDevice);
@@ -1381,9 +1469,11 @@ int lbm_batch_create(const LbmPlanDesc* common, const LbmDomainDesc* domains, in
         if (q == 19) k_flags_finalize<19><<<grid, block>>>(g);
         else k_flags_finalize<27><<<grid, block>>>(g);
         e = cudaGetLastError();
+        if (e == cudaSuccess) e = launch_wall_words(q, g, const_cast<uint32_t*>(g.walls), nullptr);
     }
     if (e == cudaSuccess) e = cudaDeviceSynchronize();
     if (e != cudaSuccess) {
+        cudaFree(b->d_walls);
         cudaFree(b->d_domains);
         cudaFree(b->d_tiles);
         delete b;
@@ -1424,6 +1514,7 @@ int lbm_batch_info(const LbmBatch* b, int64_t info[4]) {
 
 int lbm_batch_destroy(LbmBatch* b) {
     if (b == nullptr) return LBM_OK;
+    cudaFree(b->d_walls);
     cudaFree(b->d_domains);
     cudaFree(b->d_tiles);
     delete b;

@@ -125,54 +125,66 @@ __device__ __forceinline__ R load_f_out(const SweepArgs& a, int x, int y, int z,
 // Links into FixedDensity, FreeSlip, outflow and Bouzidi cells read values of other cells; inside an
 // in-place sweep those cells update concurrently, so k_boundary_prepass stores those links' values
 // where the sweep reads them before the sweep runs, as lbmpy's boundary kernel does.
+//
+// Bound by latency: a warp with one such cell waits for every load here, and with walls at the row
+// ends every warp of a cavity has one.  The directions come as one word per cell (`w`, wall_word), so
+// the bounced populations are fetched together after a single load, where a flag per neighbour cost
+// up to Q - 1 dependent round trips, one after another.
 template <class S, class R, int Q, int PAT>
 __device__ __forceinline__ void bounce_back(R (&f)[Q], const SweepArgs& a, const NbrOffsets& nb, int cell,
-                                         int x, int y, int z) {
+                                         int x, int y, int z, uint32_t w) {
     using L = Lat<Q>;
     using PA = Access<PrevPattern<PAT>::value>;
     const Grid& g = a.g;
     const S* src = static_cast<const S*>(a.src);
-    NbrOffsets fo;
-    {
-        Grid gf = g;
-        gf.sy = g.fsy; gf.sz = g.fsz;
-        fo.init(gf, x, y, z);
-    }
-    const int fcell = (x + 1) + (y + 1) * g.fsy + (z + 1) * g.fsz;
     // Interior cell indices fit 32 bits (the host bounds the field below 2^32 elements).
-    const int icell = x + g.nx * (y + g.ny * z);
+    const unsigned icell = unsigned(x) + unsigned(g.nx) * (unsigned(y) + unsigned(g.ny) * unsigned(z));
 #pragma unroll
     for (int i = 1; i < Q; ++i) {
-        const int bt = g.flags[fcell + fo.off(-L::cx(i), -L::cy(i), -L::cz(i))] & FLAG_TYPE_MASK;
-        if (bt == 0) continue;
-        // FixedDensity and per-link types: written by k_boundary_prepass (per-link types bounce back
-        // as NoSlip when the plan holds no link tables, so the pre-pass does not run)
-        if (bt >= FLAG_FIXED_DENSITY && !(bt >= FLAG_FREE_SLIP && a.link_code == nullptr && a.link_value == nullptr))
-            continue;
+        if (!((w >> i) & 1u)) continue;
         // f_out(x, inv i): where the previous step wrote direction inv(i) of this cell
         const int j = L::inv(i);
         const int off = nb.off(PA::template woff<Q>(j, 0), PA::template woff<Q>(j, 1), PA::template woff<Q>(j, 2));
-        R v = Conv<S, R>::ld(src + eidx(PA::template wslot<Q>(j) * g.sq, cell + off));
-        if (flag_is_ubb(bt)) {
-            const int u = bt - FLAG_UBB0;
-            const double* uw = a.p.ubb[u];
-            if ((a.p.ubb_link_mask >> u) & 1u)   // per-link velocity of the link x -> x - c_i (dir inv i)
-                uw = a.ubb_link_vel + (size_t(a.ubb_block[icell]) * Q + size_t(j)) * 3;
-            // compressible: the prescribed wall density, else the cell's density at the previous
-            // step, gathered before the sweep (k_ubb_density; in-place sweeps overwrite the
-            // values it is summed from)
-            const R rho = !a.p.compressible ? R(1)
-                          : a.p.ubb_density[u] > 0.0 ? R(a.p.ubb_density[u])
-                          : a.ubb_rho != nullptr ? static_cast<const R*>(a.ubb_rho)[icell] : R(1);
-            R ux = R(uw[0]), uy = R(uw[1]), uz = R(uw[2]);
-            if ((a.p.ubb_adapt_mask >> u) & 1u) {   // the equilibrium velocity of the wall
-                const R h = R(0.5) / rho;
-                ux -= h * R(a.p.force[0]); uy -= h * R(a.p.force[1]); uz -= h * R(a.p.force[2]);
-            }
-            const R cu = R(L::cx(i)) * ux + R(L::cy(i)) * uy + R(L::cz(i)) * uz;
-            v += R(6) * R(L::w(i)) * cu * rho;
+        f[i] = Conv<S, R>::ld(src + eidx(PA::template wslot<Q>(j) * g.sq, cell + off));
+    }
+    if (!(w & WALL_UBB)) return;
+    const uint32_t um = g.walls != nullptr ? g.walls[size_t(g.wall_plane) + icell] : (w | WALL_UBB_MIXED);
+    // compressible: the prescribed wall density, else the cell's density at the previous step,
+    // gathered before the sweep (k_ubb_density; in-place sweeps overwrite the values it is summed
+    // from)
+    const R rho_cell = a.ubb_rho != nullptr ? static_cast<const R*>(a.ubb_rho)[icell] : R(1);
+    R ux, uy, uz, rho;
+    auto wall = [&](int u, const double* uw) {
+        rho = !a.p.compressible ? R(1) : a.p.ubb_density[u] > 0.0 ? R(a.p.ubb_density[u]) : rho_cell;
+        ux = R(uw[0]); uy = R(uw[1]); uz = R(uw[2]);
+        if ((a.p.ubb_adapt_mask >> u) & 1u) {   // the equilibrium velocity of the wall
+            const R h = R(0.5) / rho;
+            ux -= h * R(a.p.force[0]); uy -= h * R(a.p.force[1]); uz -= h * R(a.p.force[2]);
         }
-        f[i] = v;
+    };
+    const bool each = (um & WALL_UBB_MIXED) != 0 || a.p.ubb_link_mask != 0;
+    if (!each) {                                // one wall with one velocity
+        const int u = (um >> WALL_UBB_SHIFT) & 3u;
+        wall(u, a.p.ubb[u]);
+    }
+#pragma unroll
+    for (int i = 1; i < Q; ++i) {
+        if (!((um >> i) & 1u)) continue;
+        if (each) {
+            Grid gf = g;
+            gf.sy = g.fsy;
+            gf.sz = g.fsz;
+            NbrOffsets fo;
+            fo.init(gf, x, y, z);
+            const int u = (g.flags[(x + 1) + (y + 1) * g.fsy + (z + 1) * g.fsz +
+                                   fo.off(-L::cx(i), -L::cy(i), -L::cz(i))] & FLAG_TYPE_MASK) - FLAG_UBB0;
+            if (unsigned(u) >= unsigned(MAX_UBB)) continue;
+            // per-link velocity of the link x -> x - c_i (direction inv i)
+            wall(u, ((a.p.ubb_link_mask >> u) & 1u)
+                        ? a.ubb_link_vel + (size_t(a.ubb_block[icell]) * Q + size_t(L::inv(i))) * 3 : a.p.ubb[u]);
+        }
+        const R cu = R(L::cx(i)) * ux + R(L::cy(i)) * uy + R(L::cz(i)) * uz;
+        f[i] += R(6) * R(L::w(i)) * cu * rho;
     }
 }
 
@@ -182,14 +194,14 @@ template <class S, class R, int Q, int MK, int PAT>
 __device__ __forceinline__ void sweep_cell(const SweepArgs& a, int x, int y, int z) {
     using A = Access<PAT>;
     const Grid& g = a.g;
-    // Flag first or together with the populations.  Every address below lies inside the
+    // Wall word first or together with the populations.  Every address below lies inside the
     // ghost-inclusive field whatever the cell type, so the populations can be loaded before the
-    // flag is known: a boundary cell wastes a few loads, and no cell waits for a flag round trip
-    // before its loads issue.  The specialised cumulant sweep keeps the flag first: its register
-    // budget (64 per thread for AA) does not hold the flag alongside 27 loads in flight.
-    constexpr bool flag_first = MK == MK_CUM1 || MK == MK_CUM1_MLP;
-    const int fl = (g.flags != nullptr && row_flagged(g, y, z)) ? g.flags[(x + 1) + (y + 1) * g.fsy + (z + 1) * g.fsz] : 0;
-    if (flag_first && (fl & FLAG_TYPE_MASK)) return;
+    // word is known: a boundary cell wastes a few loads, and no cell waits for a round trip
+    // before its loads issue.  The specialised cumulant sweep keeps the word first: its register
+    // budget (64 per thread for AA) does not hold it alongside 27 loads in flight.
+    constexpr bool word_first = MK == MK_CUM1 || MK == MK_CUM1_MLP;
+    const uint32_t w = wall_word<Q>(a, x, y, z);
+    if (word_first && (w & WALL_SELF)) return;
     NbrOffsets nb;
     nb.init(g, x, y, z);
     const int cell = (x + 1) + (y + 1) * g.sy + (z + 1) * g.sz;
@@ -201,8 +213,8 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs& a, int x, int y, int
         const int off = nb.off(A::template roff<Q>(i, 0), A::template roff<Q>(i, 1), A::template roff<Q>(i, 2));
         f[i] = Conv<S, R>::ld(src + eidx(A::template rslot<Q>(i) * g.sq, cell + off));
     }
-    if (!flag_first && (fl & FLAG_TYPE_MASK)) return;
-    if (fl & FLAG_NEAR_WALL) bounce_back<S, R, Q, PAT>(f, a, nb, cell, x, y, z);
+    if (!word_first && (w & WALL_SELF)) return;
+    if (w != 0) bounce_back<S, R, Q, PAT>(f, a, nb, cell, x, y, z, w);
     const R om = collide<R, Q, MK>(f, a.p);
 #pragma unroll
     for (int i = 0; i < Q; ++i) {
@@ -255,8 +267,8 @@ __global__ void __launch_bounds__(256, 2) k_sweep_zpipe(const SweepArgs a) {
     const int z1 = min(z0 + a.zc, g.nz);
     const S* src = static_cast<const S*>(a.src);
     S* dst = static_cast<S*>(a.dst);
-    auto load = [&](int z, R (&h)[Q], int& hf) {
-        hf = (g.flags != nullptr && row_flagged(g, y, z)) ? g.flags[(x + 1) + (y + 1) * g.fsy + (z + 1) * g.fsz] : 0;
+    auto load = [&](int z, R (&h)[Q], uint32_t& hw) {
+        hw = wall_word<Q>(a, x, y, z);
         NbrOffsets nb;
         nb.init(g, x, y, z);
         const int cell = (x + 1) + (y + 1) * g.sy + (z + 1) * g.sz;
@@ -267,20 +279,20 @@ __global__ void __launch_bounds__(256, 2) k_sweep_zpipe(const SweepArgs a) {
         }
     };
     R nxt[Q];
-    int nfl;
-    load(z0, nxt, nfl);
+    uint32_t nw;
+    load(z0, nxt, nw);
 #pragma unroll 1
     for (int z = z0; z < z1; ++z) {
         R f[Q];
 #pragma unroll
         for (int i = 0; i < Q; ++i) f[i] = nxt[i];
-        const int fl = nfl;
-        if (z + 1 < z1) load(z + 1, nxt, nfl);
-        if (fl & FLAG_TYPE_MASK) continue;
+        const uint32_t w = nw;
+        if (z + 1 < z1) load(z + 1, nxt, nw);
+        if (w & WALL_SELF) continue;
         NbrOffsets nb;
         nb.init(g, x, y, z);
         const int cell = (x + 1) + (y + 1) * g.sy + (z + 1) * g.sz;
-        if (fl & FLAG_NEAR_WALL) bounce_back<S, R, Q, PAT>(f, a, nb, cell, x, y, z);
+        if (w != 0) bounce_back<S, R, Q, PAT>(f, a, nb, cell, x, y, z, w);
         collide<R, Q, MK>(f, a.p);
 #pragma unroll
         for (int i = 0; i < Q; ++i) {
@@ -315,28 +327,15 @@ __device__ __forceinline__ void prefetch_cell(const SweepArgs& a, int x, int y, 
 // registers, so they are summed here first, for every pattern.
 template <class S, class R, int Q, int PAT>
 __global__ void __launch_bounds__(256) k_ubb_density(const SweepArgs a, R* rho_out) {
-    using L = Lat<Q>;
     using PA = Access<PrevPattern<PAT>::value>;
     const Grid& g = a.g;
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     const int y = blockIdx.y * blockDim.y + threadIdx.y;
     const int z = blockIdx.z;
     if (x >= g.nx || y >= g.ny) return;
-    const int fcell = (x + 1) + (y + 1) * g.fsy + (z + 1) * g.fsz;
-    const int fl = g.flags[fcell];
-    if ((fl & FLAG_TYPE_MASK) || !(fl & FLAG_NEAR_WALL)) return;
-    NbrOffsets fo;
-    {
-        Grid gf = g;
-        gf.sy = g.fsy;
-        gf.sz = g.fsz;
-        fo.init(gf, x, y, z);
-    }
-    bool moving = false;
-#pragma unroll
-    for (int i = 1; i < Q; ++i)
-        if (flag_is_ubb(g.flags[fcell + fo.off(-L::cx(i), -L::cy(i), -L::cz(i))] & FLAG_TYPE_MASK)) moving = true;
-    if (!moving) return;
+    const uint32_t w = wall_word<Q>(a, x, y, z);
+    if (!(w & WALL_UBB)) return;
+    if (g.walls == nullptr && links_from_flags<Q>(g, x, y, z, FLAG_UBB0, FLAG_UBB0 + MAX_UBB - 1) == 0) return;
     NbrOffsets nb;
     nb.init(g, x, y, z);
     const int cell = (x + 1) + (y + 1) * g.sy + (z + 1) * g.sz;
@@ -570,8 +569,12 @@ __global__ void __launch_bounds__(256) k_boundary_prepass(const SweepArgs a) {
     const int z = blockIdx.z;
     if (x >= g.nx || y >= g.ny || !row_flagged(g, y, z)) return;
     const int fcell = (x + 1) + (y + 1) * g.fsy + (z + 1) * g.fsz;
-    const int fl = g.flags[fcell];
-    if ((fl & FLAG_TYPE_MASK) || !(fl & FLAG_NEAR_WALL)) return;
+    if (g.walls != nullptr) {
+        if (!(wall_word<Q>(a, x, y, z) & (WALL_FIXED_DENSITY | WALL_PER_LINK))) return;
+    } else {
+        const int fl = g.flags[fcell];
+        if ((fl & FLAG_TYPE_MASK) || !(fl & FLAG_NEAR_WALL)) return;
+    }
     NbrOffsets fo;
     {
         Grid gf = g;

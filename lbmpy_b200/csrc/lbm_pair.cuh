@@ -131,12 +131,7 @@ __global__ void __launch_bounds__(32 * PAIR_ROWS, PairMinBlocks<S>::value) k_swe
     const S* src = static_cast<const S*>(a.src);
     S* dst = static_cast<S*>(a.dst);
 
-    int flA = 0, flB = 0;
-    if (g.flags != nullptr && row_flagged(g, y, z)) {
-        const int fc = (x0 + 1) + (y + 1) * g.fsy + (z + 1) * g.fsz;
-        flA = g.flags[fc];
-        flB = g.flags[fc + 1];
-    }
+    const uint32_t wA = wall_word<Q>(a, x0, y, z), wB = wall_word<Q>(a, x0 + 1, y, z);
 
     F2 f[Q];
 #pragma unroll
@@ -161,12 +156,12 @@ __global__ void __launch_bounds__(32 * PAIR_ROWS, PairMinBlocks<S>::value) k_swe
         f[i] = F2(va, vb);
     }
     // cells next to a boundary: per-cell fused bounce-back on the scalar path
-    if ((flA | flB) & FLAG_NEAR_WALL) {
+    if ((wA | wB) & ~WALL_SELF) {
         float ta[Q], tb[Q];
 #pragma unroll
         for (int i = 0; i < Q; ++i) { ta[i] = f[i].v.x; tb[i] = f[i].v.y; }
-        if (flA & FLAG_NEAR_WALL) bounce_back<S, float, Q, PAT>(ta, a, nbA, cellA, x0, y, z);
-        if (flB & FLAG_NEAR_WALL) bounce_back<S, float, Q, PAT>(tb, a, nbB, cellA + 1, x0 + 1, y, z);
+        if (wA & ~WALL_SELF) bounce_back<S, float, Q, PAT>(ta, a, nbA, cellA, x0, y, z, wA);
+        if (wB & ~WALL_SELF) bounce_back<S, float, Q, PAT>(tb, a, nbB, cellA + 1, x0 + 1, y, z, wB);
 #pragma unroll
         for (int i = 0; i < Q; ++i) f[i] = F2(ta[i], tb[i]);
     }
@@ -174,8 +169,8 @@ __global__ void __launch_bounds__(32 * PAIR_ROWS, PairMinBlocks<S>::value) k_swe
     // Non-fluid cells must leave their own slots as they are in AA even steps, where neighbours
     // read them (fused bounce-back): slot inv(i) is rewritten with its current value.  Pull and
     // AA odd never read what a non-fluid cell writes.
-    if (PAT == PAT_AA_EVEN && ((flA | flB) & FLAG_TYPE_MASK)) {
-        const bool keepA = (flA & FLAG_TYPE_MASK) != 0, keepB = (flB & FLAG_TYPE_MASK) != 0;
+    if (PAT == PAT_AA_EVEN && ((wA | wB) & WALL_SELF)) {
+        const bool keepA = (wA & WALL_SELF) != 0, keepB = (wB & WALL_SELF) != 0;
 #pragma unroll
         for (int i = 0; i < Q; ++i) {
             const S* q = src + eidx(L::inv(i) * g.sq, cellA);

@@ -77,11 +77,10 @@ __global__ void __launch_bounds__(32 * QUAD_ROWS, 4) k_sweep_quad(const SweepArg
     const S* src = static_cast<const S*>(a.src);
     S* dst = static_cast<S*>(a.dst);
 
-    int fl[4] = {0, 0, 0, 0};
+    uint32_t w[4] = {0, 0, 0, 0};
     if (g.flags != nullptr && row_flagged(g, y, z)) {
-        const int fc = (x0 + 1) + (y + 1) * g.fsy + (z + 1) * g.fsz;
 #pragma unroll
-        for (int k = 0; k < 4; ++k) fl[k] = g.flags[fc + k];
+        for (int k = 0; k < 4; ++k) w[k] = wall_word<Q>(a, x0 + k, y, z);
     }
 
     F2 f0[Q], f1[Q];     // cells (x0, x0+1) and (x0+2, x0+3)
@@ -108,10 +107,10 @@ __global__ void __launch_bounds__(32 * QUAD_ROWS, 4) k_sweep_quad(const SweepArg
         f1[i] = F2(v[2], v[3]);
     }
     // cells next to a boundary: per-cell fused bounce-back on the scalar path
-    if ((fl[0] | fl[1] | fl[2] | fl[3]) & FLAG_NEAR_WALL) {
+    if ((w[0] | w[1] | w[2] | w[3]) & ~WALL_SELF) {
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            if (!(fl[k] & FLAG_NEAR_WALL)) continue;
+            if (!(w[k] & ~WALL_SELF)) continue;
             float t[Q];
 #pragma unroll
             for (int i = 0; i < Q; ++i) {
@@ -120,7 +119,7 @@ __global__ void __launch_bounds__(32 * QUAD_ROWS, 4) k_sweep_quad(const SweepArg
             }
             NbrOffsets nb;
             nb.init(g, x0 + k, y, z);
-            bounce_back<S, float, Q, PAT>(t, a, nb, cellA + k, x0 + k, y, z);
+            bounce_back<S, float, Q, PAT>(t, a, nb, cellA + k, x0 + k, y, z, w[k]);
 #pragma unroll
             for (int i = 0; i < Q; ++i) {
                 F2& h = k < 2 ? f0[i] : f1[i];
@@ -132,14 +131,14 @@ __global__ void __launch_bounds__(32 * QUAD_ROWS, 4) k_sweep_quad(const SweepArg
     collide2<float, Q, MK>(f1, a.p);
     // Non-fluid cells leave their own slots as they are in AA even steps (neighbours read them in
     // the fused bounce-back): slot inv(i) is rewritten with its current value.
-    if (PAT == PAT_AA_EVEN && ((fl[0] | fl[1] | fl[2] | fl[3]) & FLAG_TYPE_MASK)) {
+    if (PAT == PAT_AA_EVEN && ((w[0] | w[1] | w[2] | w[3]) & WALL_SELF)) {
 #pragma unroll
         for (int i = 0; i < Q; ++i) {
             const S* q = src + eidx(L::inv(i) * g.sq, cellA);
-            if (fl[0] & FLAG_TYPE_MASK) f0[i].v.x = Conv<S, float>::ld(q);
-            if (fl[1] & FLAG_TYPE_MASK) f0[i].v.y = Conv<S, float>::ld(q + 1);
-            if (fl[2] & FLAG_TYPE_MASK) f1[i].v.x = Conv<S, float>::ld(q + 2);
-            if (fl[3] & FLAG_TYPE_MASK) f1[i].v.y = Conv<S, float>::ld(q + 3);
+            if (w[0] & WALL_SELF) f0[i].v.x = Conv<S, float>::ld(q);
+            if (w[1] & WALL_SELF) f0[i].v.y = Conv<S, float>::ld(q + 1);
+            if (w[2] & WALL_SELF) f1[i].v.x = Conv<S, float>::ld(q + 2);
+            if (w[3] & WALL_SELF) f1[i].v.y = Conv<S, float>::ld(q + 3);
         }
     }
 

@@ -11,7 +11,7 @@
 // tile's edge cell pulls from outside the segment (x = xs - 1 or xs + w, with the periodic wrap)
 // is copied into the pad next to the segment by the same asynchronous copies (4 / 8 bytes; for
 // 16-bit storage the aligned 4-byte word holding it, whose other half lies in the row or in its
-// padding).  Each cell's flag is loaded one tile ahead.  Writes go straight to global memory.
+// padding).  Each cell's wall word is loaded one tile ahead.  Writes go straight to global memory.
 //
 // Every wait on a barrier is bounded (SweepArgs::stage_wait_ns, default STAGED_WAIT_NS); a CTA
 // whose stage does not complete sets
@@ -221,14 +221,13 @@ __global__ void __launch_bounds__(W) k_sweep_staged(const SweepArgs a, const int
         staged::copies_arrive(bar);
         staged::arrive(bar);
     };
-    auto flag_of = [&](const StagedTile& t) -> int {
-        if (g.flags == nullptr || tid >= t.w || !row_flagged(g, t.y, t.z)) return 0;
-        return g.flags[(t.xs + tid + 1) + (t.y + 1) * g.fsy + (t.z + 1) * g.fsz];
+    auto word_of = [&](const StagedTile& t) -> uint32_t {
+        return tid < t.w ? wall_word<Q>(a, t.xs + tid, t.y, t.z) : 0u;
     };
 
     const int npro = min(ns, mine);
     for (int k = 0; k < npro; ++k) issue(hdr[k], k);
-    int fl = mine > 0 ? flag_of(hdr[0]) : 0;
+    uint32_t w = mine > 0 ? word_of(hdr[0]) : 0;
 
     for (int k = 0; k < mine; ++k) {
         const int s = k % ns;
@@ -262,14 +261,14 @@ __global__ void __launch_bounds__(W) k_sweep_staged(const SweepArgs a, const int
                 }
             }
         }
-        const int fl_next = k + 1 < mine ? flag_of(hdr[(k + 1) % ns]) : 0;
+        const uint32_t w_next = k + 1 < mine ? word_of(hdr[(k + 1) % ns]) : 0;
 
-        if (tid < t.w && !(fl & FLAG_TYPE_MASK)) {
+        if (tid < t.w && !(w & WALL_SELF)) {
             const int x = t.xs + tid;
             NbrOffsets nb;
             nb.init(g, x, t.y, t.z);
             const int cell = (x + 1) + (t.y + 1) * g.sy + (t.z + 1) * g.sz;
-            if (fl & FLAG_NEAR_WALL) bounce_back<S, R, Q, PAT>(f, a, nb, cell, x, t.y, t.z);
+            if (w != 0) bounce_back<S, R, Q, PAT>(f, a, nb, cell, x, t.y, t.z, w);
             const R om = collide<R, Q, MK>(f, a.p);
 #pragma unroll
             for (int i = 0; i < Q; ++i) {
@@ -278,7 +277,7 @@ __global__ void __launch_bounds__(W) k_sweep_staged(const SweepArgs a, const int
             }
             if (a.omega_out != nullptr) a.omega_out[x + g.nx * (t.y + (long long)g.ny * t.z)] = (float)om;
         }
-        fl = fl_next;
+        w = w_next;
     }
 }
 
