@@ -16,6 +16,7 @@
 #include "../../include/lbm_b200.h"
 #include "lbm_closure.cuh"
 #include "lbm_dispatch.h"
+#include "lbm_reduce.cuh"
 
 using namespace lbm;
 
@@ -1023,7 +1024,7 @@ int lbm_reduce_conserved(const LbmPlan* p, const void* pdfs, const int64_t strid
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     cudaError_t e = L(a, p->red_blocks, p->partial, s);
     if (e != cudaSuccess) return cuda_fail(e, "reduction launch");
-    k_reduce_finish<<<1, 32, 0, s>>>(p->partial, p->red_blocks, p->red_out);
+    k_reduce_finish<<<1, 160, 0, s>>>(p->partial, p->red_blocks, p->red_out);
     e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(e, "reduction finish launch");
     e = cudaMemcpyAsync(out, p->red_out, 5 * sizeof(double), cudaMemcpyDeviceToHost, s);
@@ -1603,7 +1604,7 @@ extern "C" int lbm_reduce_conserved_noalloc(const LbmPlanDesc* desc, const void*
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     e = L(a, blocks, partial, s);
     if (e != cudaSuccess) return cuda_fail(e, "reduction launch");
-    k_reduce_finish<<<1, 32, 0, s>>>(partial, blocks, result);
+    k_reduce_finish<<<1, 160, 0, s>>>(partial, blocks, result);
     e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(e, "reduction finish launch");
     e = cudaMemcpyAsync(out, result, 5 * sizeof(double), cudaMemcpyDeviceToHost, s);
