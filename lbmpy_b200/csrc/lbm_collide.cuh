@@ -29,8 +29,8 @@ template <int Q, class R> struct Macro {
     R drho, rho, rho_ref, ux, uy, uz;
 };
 
-template <int Q, class R>
-__device__ __forceinline__ Macro<Q, R> conserved(const R (&f)[Q], const Physics& p, bool eq_shift) {
+template <int Q, class R, class P>
+__device__ __forceinline__ Macro<Q, R> conserved(const R (&f)[Q], const P& p, bool eq_shift) {
     using L = Lat<Q>;
     R d = 0, jx = 0, jy = 0, jz = 0;
 #pragma unroll
@@ -48,15 +48,15 @@ __device__ __forceinline__ Macro<Q, R> conserved(const R (&f)[Q], const Physics&
     m.ux = jx * inv; m.uy = jy * inv; m.uz = jz * inv;
     if (eq_shift) {
         const R h = R(0.5) * inv;
-        m.ux += h * R(p.force[0]); m.uy += h * R(p.force[1]); m.uz += h * R(p.force[2]);
+        m.ux += h * p_force<R>(p, 0); m.uy += h * p_force<R>(p, 1); m.uz += h * p_force<R>(p, 2);
     }
     return m;
 }
 
 // Smagorinsky rate from the non-equilibrium stress.  f_eq's second raw moments are
 // rho_f*u_a*u_b + delta_ab*drho/3 for every method here (they are matched moments).
-template <int Q, class R>
-__device__ __forceinline__ R smagorinsky_rate(const R (&f)[Q], const Macro<Q, R>& m, const Physics& p) {
+template <int Q, class R, class P>
+__device__ __forceinline__ R smagorinsky_rate(const R (&f)[Q], const Macro<Q, R>& m, const P& p) {
     using L = Lat<Q>;
     R sxx = 0, syy = 0, szz = 0, sxy = 0, sxz = 0, syz = 0;
 #pragma unroll
@@ -78,17 +78,17 @@ __device__ __forceinline__ R smagorinsky_rate(const R (&f)[Q], const Macro<Q, R>
     const R pyz = syz - rf * m.uy * m.uz;
     const R s2 = pxx * pxx + pyy * pyy + pzz * pzz + R(2) * (pxy * pxy + pxz * pxz + pyz * pyz);
     const R pi = sqrt(R(2) * s2) / m.rho_ref;
-    const R tau0 = R(p.tau0);
-    return R(2) / (tau0 + sqrt(R(p.sgs_c18) * pi + tau0 * tau0));
+    const R tau0 = p_tau0<R>(p);
+    return R(2) / (tau0 + sqrt(p_c18<R>(p) * pi + tau0 * tau0));
 }
 
 // ------------------------------------------------------------------ SRT / TRT
-template <int Q, class R>
-__device__ __forceinline__ R collide_pop(R (&f)[Q], const Physics& p) {
+template <int Q, class R, class P>
+__device__ __forceinline__ R collide_pop(R (&f)[Q], const P& p) {
     using L = Lat<Q>;
     const bool shift = p.force_model == FM_GUO || p.force_model == FM_CENTRAL;
     const Macro<Q, R> m = conserved<Q, R>(f, p, shift);
-    R wp = R(p.rates[0]), wm = R(p.rates[1]);
+    R wp = p_rate<R>(p, 0), wm = p_rate<R>(p, 1);
     if (p.sgs == 1) {
         const R om = smagorinsky_rate<Q, R>(f, m, p);
         if (p.sgs_mask & 1u) wp = om;
@@ -99,7 +99,7 @@ __device__ __forceinline__ R collide_pop(R (&f)[Q], const Physics& p) {
     const R uxy = m.ux * m.uy, uxz = m.ux * m.uz, uyz = m.uy * m.uz;
     const bool cont = p.continuous_eq != 0;
     const bool has_force = p.force_model == FM_GUO || p.force_model == FM_SIMPLE || p.force_model == FM_LUO;
-    const R Fx = R(p.force[0]), Fy = R(p.force[1]), Fz = R(p.force[2]);
+    const R Fx = p_force<R>(p, 0), Fy = p_force<R>(p, 1), Fz = p_force<R>(p, 2);
     const R uF = m.ux * Fx + m.uy * Fy + m.uz * Fz;
     R fe_scale = R(1), fo_scale = R(1), fe_on = R(1);
     if (p.force_model == FM_GUO) { fe_scale = R(1) - R(0.5) * wp; fo_scale = R(1) - R(0.5) * wm; }
@@ -147,8 +147,8 @@ __device__ __forceinline__ R collide_pop(R (&f)[Q], const Physics& p) {
 }
 
 // ------------------------------------------------------------------ MRT (raw moment space)
-template <int Q, class R>
-__device__ __forceinline__ R collide_mrt(R (&f)[Q], const Physics& p) {
+template <int Q, class R, class P>
+__device__ __forceinline__ R collide_mrt(R (&f)[Q], const P& p) {
     using L = Lat<Q>;
     const bool shift = p.force_model == FM_GUO || p.force_model == FM_CENTRAL;
     const Macro<Q, R> m = conserved<Q, R>(f, p, shift);
@@ -160,7 +160,7 @@ __device__ __forceinline__ R collide_mrt(R (&f)[Q], const Physics& p) {
     // Moments of the force populations (Luo and Guo: w_i (9 (c.F)(c.u) + 3 c.F - 3 u.F); Simple:
     // 3 w_i c.F) in closed form: the even rows see 9 sum_ab T_ab F_a u_b - 3 (u.F) S, the odd rows
     // 3 sum_a B_a F_a (tables generated from the basis).
-    const R Fx = R(p.force[0]), Fy = R(p.force[1]), Fz = R(p.force[2]);
+    const R Fx = p_force<R>(p, 0), Fy = p_force<R>(p, 1), Fz = p_force<R>(p, 2);
     const bool simple = p.force_model == FM_SIMPLE;
     const R FU[6] = {Fx * m.ux, Fy * m.uy, Fz * m.uz, Fx * m.uy + Fy * m.ux, Fx * m.uz + Fz * m.ux,
                      Fy * m.uz + Fz * m.uy};
@@ -200,7 +200,7 @@ __device__ __forceinline__ R collide_mrt(R (&f)[Q], const Physics& p) {
 #pragma unroll
         for (int a = 0; a < 6; ++a) quad = cmad(quad, L::mquad(k, a), uu[a]);
         const R meq = cmad(rf * (lin + quad), L::p0(k), m.drho);
-        R r = R(p.rates[k]);
+        R r = p_rate<R>(p, k);
         if (p.sgs == 1 && ((p.sgs_mask >> k) & 1u)) r = om_sgs;
         R d = r * (meq - mk);
         if (has_force) {
@@ -267,23 +267,24 @@ __device__ __forceinline__ void chimera_forward(R (&g)[27], R u, int stride, int
 // Backward: central moments about u -> populations, axis by axis.
 template <class R>
 __device__ __forceinline__ void chimera_backward(R (&g)[27], R u, int stride, int s1, int s2) {
+    const R hu = R(0.5) * u, u2 = R(2) * u, uu = u * u;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
 #pragma unroll
         for (int b = 0; b < 3; ++b) {
             const int base = a * s1 + b * s2;
             const R k0 = g[base], k1 = g[base + stride], k2 = g[base + 2 * stride];
-            const R m1 = k1 + u * k0;
-            const R m2 = k2 + R(2) * u * k1 + u * u * k0;
-            g[base] = R(0.5) * (m2 - m1);
+            const R h1 = R(0.5) * k1 + hu * k0;            // half the first and the second moment
+            const R m2 = k2 + u2 * k1 + uu * k0;
+            g[base] = R(0.5) * m2 - h1;
             g[base + stride] = k0 - m2;
-            g[base + 2 * stride] = R(0.5) * (m2 + m1);
+            g[base + 2 * stride] = R(0.5) * m2 + h1;
         }
     }
 }
 
-template <class R>
-__device__ __forceinline__ R collide_cum(R (&f)[27], const Physics& p) {
+template <class R, class P>
+__device__ __forceinline__ R collide_cum(R (&f)[27], const P& p) {
     using L = Lat<27>;
     const bool cm_force = p.force_model == FM_CENTRAL;
     const Macro<27, R> m = conserved<27, R>(f, p, cm_force);
@@ -339,7 +340,7 @@ __device__ __forceinline__ R collide_cum(R (&f)[27], const Physics& p) {
 
     // ---- relaxation of the polynomial cumulants (group rates from the plan)
     auto rate = [&](int idx) -> R {
-        R r = R(p.rates[idx]);
+        R r = p_rate<R>(p, idx);
         if (p.sgs == 1 && ((p.sgs_mask >> idx) & 1u)) r = om_sgs;
         return r;
     };
@@ -352,7 +353,7 @@ __device__ __forceinline__ R collide_cum(R (&f)[27], const Physics& p) {
     R Ps_b = P_b + w_b * (rho - P_b);
     const R c110 = k110 - w_xy * k110, c101 = k101 - w_xz * k101, c011 = k011 - w_yz * k011;
     if (p.galilean) {
-        const R o1 = R(p.rates[7]), o2 = R(p.rates[9]);   // base rates, not the SGS-adapted ones
+        const R o1 = p_rate<R>(p, 7), o2 = p_rate<R>(p, 9);   // base rates, not the SGS-adapted ones
         const R h = R(0.5) * irho;
         const R Dx = -o1 * h * (R(2) * k200 - k020 - k002) - o2 * h * (k200 + k020 + k002 - rho);
         const R Dy = Dx + R(3) * o1 * h * (k200 - k020);
@@ -396,19 +397,19 @@ __device__ __forceinline__ R collide_cum(R (&f)[27], const Physics& p) {
         // correction terms of the fourth-order polynomial cumulants from velocity-derivative
         // estimates of the pre-collision second-order cumulants (Geier et al. 2017, eq. 44-49;
         // fourth_order_correction.py:100-145)
-        const R o1 = R(p.rates[4]), o2 = R(p.rates[9]);
+        const R o1 = p_rate<R>(p, 4), o2 = p_rate<R>(p, 9);
         const R h = R(0.5) * irho;
         const R Dx = -o1 * h * (R(2) * k200 - k020 - k002) - o2 * h * (k200 + k020 + k002 - rho);
         const R Dy = Dx + R(3) * o1 * h * (k200 - k020);
         const R Dz = Dx + R(3) * o1 * h * (k200 - k002);
         const R g = (R(1) / o1 - R(0.5)) * rho;
         const R ca = g * R(p.foc_a), cb = g * R(p.foc_b) * R(-1.0 / 3.0) * R(-3) * o1 * irho;
-        q1 += R(2.0 / 3.0) * R(p.rates[17]) * ca * (Dx - R(2) * Dy + Dz);
-        q2 += R(2.0 / 3.0) * R(p.rates[17]) * ca * (Dx + Dy - R(2) * Dz);
-        q3 += R(-4.0 / 3.0) * R(p.rates[19]) * ca * (Dx + Dy + Dz);
-        C211s += R(p.rates[20]) * cb * k011;
-        C121s += R(p.rates[20]) * cb * k101;
-        C112s += R(p.rates[20]) * cb * k110;
+        q1 += R(2.0 / 3.0) * p_rate<R>(p, 17) * ca * (Dx - R(2) * Dy + Dz);
+        q2 += R(2.0 / 3.0) * p_rate<R>(p, 17) * ca * (Dx + Dy - R(2) * Dz);
+        q3 += R(-4.0 / 3.0) * p_rate<R>(p, 19) * ca * (Dx + Dy + Dz);
+        C211s += p_rate<R>(p, 20) * cb * k011;
+        C121s += p_rate<R>(p, 20) * cb * k101;
+        C112s += p_rate<R>(p, 20) * cb * k110;
     }
     const R C220s = (q3 + q1 + q2) * R(1.0 / 3.0);
     const R C202s = (q3 - q1) * R(1.0 / 3.0);
@@ -442,9 +443,9 @@ __device__ __forceinline__ R collide_cum(R (&f)[27], const Physics& p) {
                   R(8) * c110 * c101 * c011) * irho * irho;
     // symmetric forcing, second half: first-order central moments become F/2
     if (cm_force) {
-        K(1, 0, 0) = R(0.5) * R(p.force[0]);
-        K(0, 1, 0) = R(0.5) * R(p.force[1]);
-        K(0, 0, 1) = R(0.5) * R(p.force[2]);
+        K(1, 0, 0) = R(0.5) * p_force<R>(p, 0);
+        K(0, 1, 0) = R(0.5) * p_force<R>(p, 1);
+        K(0, 0, 1) = R(0.5) * p_force<R>(p, 2);
     }
 #undef K
 #pragma unroll
@@ -458,7 +459,7 @@ __device__ __forceinline__ R collide_cum(R (&f)[27], const Physics& p) {
     chimera_backward(k, uz, 1, 9, 3);
 #pragma unroll
     for (int i = 0; i < 27; ++i) f[i] = k[cube<27>(i)];
-    return p.sgs == 1 ? om_sgs : R(p.rates[4]);
+    return p.sgs == 1 ? om_sgs : p_rate<R>(p, 4);
 }
 
 // D3Q27 central-moment method (methods/momentbased/centralmomentbasedmethod.py:296-394): the
@@ -467,8 +468,8 @@ __device__ __forceinline__ R collide_cum(R (&f)[27], const Physics& p) {
 // Gaussian of variance 1/3; the force model's population term (Simple, Luo, Guo) enters in
 // central-moment space, scaled by (1 - omega/2) per moment for Guo (forcemodels.py:201-203,
 // 261-263, 300-306).  Compressible, zero-centred storage with the lattice-weight background.
-template <class R>
-__device__ __forceinline__ R collide_cm(R (&f)[27], const Physics& p) {
+template <class R, class P>
+__device__ __forceinline__ R collide_cm(R (&f)[27], const P& p) {
     using L = Lat<27>;
     const bool guo = p.force_model == FM_GUO;
     const bool forced = p.force_model == FM_GUO || p.force_model == FM_LUO || p.force_model == FM_SIMPLE;
@@ -495,7 +496,7 @@ __device__ __forceinline__ R collide_cm(R (&f)[27], const Physics& p) {
 #pragma unroll
     for (int i = 0; i < 27; ++i) g[i] = R(0);
     if (forced) {
-        const R Fx = R(p.force[0]), Fy = R(p.force[1]), Fz = R(p.force[2]);
+        const R Fx = p_force<R>(p, 0), Fy = p_force<R>(p, 1), Fz = p_force<R>(p, 2);
 #pragma unroll
         for (int i = 0; i < 27; ++i) {
             const R cF = R(L::cx(i)) * Fx + R(L::cy(i)) * Fy + R(L::cz(i)) * Fz;
@@ -512,7 +513,7 @@ __device__ __forceinline__ R collide_cm(R (&f)[27], const Physics& p) {
 #define G(a, b, c) g[(a) * 9 + (b) * 3 + (c)]
     // post = pre + omega (eq - pre) + corr * force, corr = 1 - omega/2 for Guo
     auto relax = [&](int idx, R pre, R eq, R frc) -> R {
-        const R w = R(p.rates[idx]);
+        const R w = p_rate<R>(p, idx);
         return pre + w * (eq - pre) + (guo ? R(1) - R(0.5) * w : R(1)) * frc;
     };
     const R third = R(1.0 / 3.0);
@@ -573,7 +574,7 @@ __device__ __forceinline__ R collide_cm(R (&f)[27], const Physics& p) {
     chimera_backward(k, uz, 1, 9, 3);
 #pragma unroll
     for (int i = 0; i < 27; ++i) f[i] = k[cube<27>(i)];
-    return R(p.rates[4]);
+    return p_rate<R>(p, 4);
 }
 
 // D3Q27 cumulant when every cumulant of third and higher order relaxes with rate 1 (lbmpy's
@@ -586,8 +587,8 @@ __device__ __forceinline__ R collide_cm(R (&f)[27], const Physics& p) {
 // CLOSURE: the shear rate comes from an eddy viscosity nu_t(Pi_xx, Pi_yy, Pi_zz, Pi_xy, Pi_xz,
 // Pi_yz, rho, ux, uy, uz) evaluated on the same non-equilibrium stress the Smagorinsky branch uses
 // (the learned closure, lbm_closure.cuh), as omega = 1 / (tau0 + 3 nu_t).
-template <class R, bool CLOSURE = false, class NU = int>
-__device__ __forceinline__ R collide_cum_ho1(R (&f)[27], const Physics& p, const NU& nu_t = NU()) {
+template <class R, bool CLOSURE = false, class NU = int, class P = Physics>
+__device__ __forceinline__ R collide_cum_ho1(R (&f)[27], const P& p, const NU& nu_t = NU()) {
     // raw moments of f~ (no shift) on the velocity cube: m[a*9 + b*3 + c]
     R m[27];
 #pragma unroll
@@ -621,7 +622,7 @@ __device__ __forceinline__ R collide_cum_ho1(R (&f)[27], const Physics& p, const
     const R rho = R(1) + drho, irho = R(1) / rho;
     const bool cm_force = p.force_model == FM_CENTRAL;
     R ux = M_(1, 0, 0) * irho, uy = M_(0, 1, 0) * irho, uz = M_(0, 0, 1) * irho;
-    const R hx = R(0.5) * R(p.force[0]), hy = R(0.5) * R(p.force[1]), hz = R(0.5) * R(p.force[2]);
+    const R hx = R(0.5) * p_force<R>(p, 0), hy = R(0.5) * p_force<R>(p, 1), hz = R(0.5) * p_force<R>(p, 2);
     if (cm_force) { ux += hx * irho; uy += hy * irho; uz += hz * irho; }
     const R uxx = ux * ux, uyy = uy * uy, uzz = uz * uz;
     // second-order central moments of the full PDFs minus rho/3 (diagonal) -- small numbers:
@@ -637,24 +638,24 @@ __device__ __forceinline__ R collide_cum_ho1(R (&f)[27], const Physics& p, const
     R om_sgs = R(0);
     if (CLOSURE || p.sgs == 1) {
         // Pi_neq from the central moments: raw second moments minus their equilibrium values
-        const R pxx = a0 - ux * R(p.force[0]) * R(cm_force ? 1 : 0);
-        const R pyy = b0 - uy * R(p.force[1]) * R(cm_force ? 1 : 0);
-        const R pzz = c0 - uz * R(p.force[2]) * R(cm_force ? 1 : 0);
-        const R fxy = cm_force ? R(0.5) * (ux * R(p.force[1]) + uy * R(p.force[0])) : R(0);
-        const R fxz = cm_force ? R(0.5) * (ux * R(p.force[2]) + uz * R(p.force[0])) : R(0);
-        const R fyz = cm_force ? R(0.5) * (uy * R(p.force[2]) + uz * R(p.force[1])) : R(0);
+        const R pxx = a0 - ux * p_force<R>(p, 0) * R(cm_force ? 1 : 0);
+        const R pyy = b0 - uy * p_force<R>(p, 1) * R(cm_force ? 1 : 0);
+        const R pzz = c0 - uz * p_force<R>(p, 2) * R(cm_force ? 1 : 0);
+        const R fxy = cm_force ? R(0.5) * (ux * p_force<R>(p, 1) + uy * p_force<R>(p, 0)) : R(0);
+        const R fxz = cm_force ? R(0.5) * (ux * p_force<R>(p, 2) + uz * p_force<R>(p, 0)) : R(0);
+        const R fyz = cm_force ? R(0.5) * (uy * p_force<R>(p, 2) + uz * p_force<R>(p, 1)) : R(0);
         const R pxy = k110 - fxy, pxz = k101 - fxz, pyz = k011 - fyz;
         if constexpr (CLOSURE) {
-            om_sgs = R(1) / (R(p.tau0) + R(3) * nu_t(pxx, pyy, pzz, pxy, pxz, pyz, rho, ux, uy, uz));
+            om_sgs = R(1) / (p_tau0<R>(p) + R(3) * nu_t(pxx, pyy, pzz, pxy, pxz, pyz, rho, ux, uy, uz));
         } else {
             const R s2 = pxx * pxx + pyy * pyy + pzz * pzz + R(2) * (pxy * pxy + pxz * pxz + pyz * pyz);
             const R pi = sqrt(R(2) * s2) * irho;
-            const R tau0 = R(p.tau0);
-            om_sgs = R(2) / (tau0 + sqrt(R(p.sgs_c18) * pi + tau0 * tau0));
+            const R tau0 = p_tau0<R>(p);
+            om_sgs = R(2) / (tau0 + sqrt(p_c18<R>(p) * pi + tau0 * tau0));
         }
     }
     auto rate = [&](int idx) -> R {
-        R r = R(p.rates[idx]);
+        R r = p_rate<R>(p, idx);
         if ((CLOSURE || p.sgs == 1) && ((p.sgs_mask >> idx) & 1u)) r = om_sgs;
         return r;
     };
@@ -663,7 +664,7 @@ __device__ __forceinline__ R collide_cum_ho1(R (&f)[27], const Physics& p, const
     R D2 = (a0 - c0) * (R(1) - w_d2);
     R Sd = (a0 + b0 + c0) * (R(1) - w_b);   // (sum of diagonal second cumulants) - rho
     if (p.galilean) {
-        const R o1 = R(p.rates[7]), o2 = R(p.rates[9]);
+        const R o1 = p_rate<R>(p, 7), o2 = p_rate<R>(p, 9);
         const R h = R(0.5) * irho;
         // c_xx = rho/3 + a0: 2cxx - cyy - czz = 2a0 - b0 - c0; cxx + cyy + czz - rho = a0 + b0 + c0
         const R Dx = -o1 * h * (R(2) * a0 - b0 - c0) - o2 * h * (a0 + b0 + c0);
@@ -725,7 +726,7 @@ __device__ __forceinline__ R collide_cum_ho1(R (&f)[27], const Physics& p, const
     chimera_backward(d, uz, 1, 9, 3);
 #pragma unroll
     for (int i = 0; i < 27; ++i) f[i] = d[cube<27>(i)];
-    return (CLOSURE || p.sgs == 1) ? om_sgs : R(p.rates[4]);
+    return (CLOSURE || p.sgs == 1) ? om_sgs : p_rate<R>(p, 4);
 }
 
 // ------------------------------------------------------------------ equilibria (setter)

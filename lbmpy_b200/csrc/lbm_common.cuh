@@ -2,6 +2,7 @@
 // conversions and the by-value argument block every kernel receives.
 #pragma once
 #include <cstdint>
+#include <type_traits>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -193,6 +194,33 @@ struct Physics {
     double foc_a, foc_b;          // its parameters a and b (Geier et al. 2017, eq. 115-116)
 };
 
+// What a sweep receives: Physics and FP32 copies of what every FP32 cell reads.  A cell that converts
+// the doubles itself spends a double-to-float conversion on each, on a quarter-rate pipe.
+struct SweepPhysics : Physics {
+    float rates32[27], force32[3], sgs_c18_32, tau0_32;
+    SweepPhysics& operator=(const Physics& p) {
+        static_cast<Physics&>(*this) = p;
+        for (int k = 0; k < 27; ++k) rates32[k] = float(p.rates[k]);
+        for (int k = 0; k < 3; ++k) force32[k] = float(p.force[k]);
+        sgs_c18_32 = float(p.sgs_c18);
+        tau0_32 = float(p.tau0);
+        return *this;
+    }
+};
+
+template <class R> LBM_HD R p_rate(const Physics& p, int k) { return R(p.rates[k]); }
+template <class R> LBM_HD R p_force(const Physics& p, int k) { return R(p.force[k]); }
+template <class R> LBM_HD R p_c18(const Physics& p) { return R(p.sgs_c18); }
+template <class R> LBM_HD R p_tau0(const Physics& p) { return R(p.tau0); }
+template <class R> LBM_HD R p_pick(double d, float f) {
+    if constexpr (std::is_same<R, double>::value) return d;
+    else return R(f);
+}
+template <class R> LBM_HD R p_rate(const SweepPhysics& p, int k) { return p_pick<R>(p.rates[k], p.rates32[k]); }
+template <class R> LBM_HD R p_force(const SweepPhysics& p, int k) { return p_pick<R>(p.force[k], p.force32[k]); }
+template <class R> LBM_HD R p_c18(const SweepPhysics& p) { return p_pick<R>(p.sgs_c18, p.sgs_c18_32); }
+template <class R> LBM_HD R p_tau0(const SweepPhysics& p) { return p_pick<R>(p.tau0, p.tau0_32); }
+
 struct Grid {
     int nx, ny, nz;        // interior cells
     int sy, sz;            // element strides of y and z (x stride is 1)
@@ -212,7 +240,7 @@ struct Grid {
 
 struct SweepArgs {
     Grid g;
-    Physics p;
+    SweepPhysics p;
     const void* src;
     void* dst;
     float* omega_out;      // optional per-cell effective shear rate (interior, x fastest)

@@ -74,18 +74,54 @@ template <int PAT> struct PrevPattern {
 // sweep, lbm_q27_closure.cu.
 template <class R> struct ClosureNu;
 
-template <class R, int Q, int MK>
-__device__ __forceinline__ R collide(R (&f)[Q], const Physics& p) {
-    if constexpr (MK == MK_POP) return collide_pop<Q, R>(f, p);
-    else if constexpr (MK == MK_MRT) return collide_mrt<Q, R>(f, p);
-    else if constexpr (MK == MK_CUM1) return collide_cum_ho1<R>(f, p);
-    else if constexpr (MK == MK_CUM1_MLP) return collide_cum_ho1<R, true>(f, p, ClosureNu<R>{});
-    else if constexpr (MK == MK_CM) return collide_cm<R>(f, p);
-    else return collide_cum<R>(f, p);
+// The collision operator of a method kind; returns the effective shear rate.
+template <int MK> struct Collision;
+#define LBM_COLLISION(MK, CALL)                                                     \
+    template <> struct Collision<MK> {                                              \
+        template <int Q, class R, class P>                                          \
+        __device__ __forceinline__ static R run(R (&f)[Q], const P& p) { return CALL; } \
+    };
+LBM_COLLISION(MK_POP, (collide_pop<Q, R>(f, p)))
+LBM_COLLISION(MK_MRT, (collide_mrt<Q, R>(f, p)))
+LBM_COLLISION(MK_CUM, (collide_cum<R>(f, p)))
+LBM_COLLISION(MK_CUM1, (collide_cum_ho1<R>(f, p)))
+LBM_COLLISION(MK_CUM1_MLP, (collide_cum_ho1<R, true>(f, p, ClosureNu<R>{})))
+LBM_COLLISION(MK_CM, (collide_cm<R>(f, p)))
+#undef LBM_COLLISION
+
+template <class R, int Q, int MK, class P>
+__device__ __forceinline__ R collide(R (&f)[Q], const P& p) { return Collision<MK>::template run<Q, R>(f, p); }
+
+// Address of (slot, cell + offset) of a field.  The slot part is the same for every thread, the cell
+// part fits 32 bits in bytes too (the host bounds Q slots to 2^32 elements), so that one register
+// holds the offset that several slots share and the rest stays in uniform registers.
+template <class S> __device__ __forceinline__ S* at(S* field, unsigned slot_off, int cell_off) {
+    using C = typename std::conditional<std::is_const<S>::value, const char, char>::type;
+    return reinterpret_cast<S*>(reinterpret_cast<C*>(field + size_t(slot_off)) +
+                                size_t(unsigned(cell_off) * unsigned(sizeof(S))));
 }
 
-// Element index of (slot, cell + offset) relative to the field base; 32-bit (host-checked).
-__device__ __forceinline__ unsigned eidx(unsigned slot_off, int cell_off) { return slot_off + (unsigned)cell_off; }
+// The slots of a field in order.  With the field's strides in kernel parameters a slot's address is
+// uniform arithmetic; read from shared memory they are ordinary registers, where the compiler keeps the
+// products of all slots from the loads to the stores and spills: there the address is walked, hidden
+// from it step by step.
+template <class S, bool WALK> struct Slots {
+    S* field;
+    unsigned sq;
+    __device__ __forceinline__ Slots(S* f, unsigned stride) : field(f), sq(stride) {}
+    // Address of (slot, cell offset); slots must be taken in ascending order, without gaps from 0.
+    __device__ __forceinline__ S* operator()(int slot, int cell_off) {
+        if constexpr (WALK) {
+            if (slot > 0) {
+                field += sq;
+                asm volatile("" : "+l"(field));
+            }
+            return at(field, 0u, cell_off);
+        } else {
+            return at(field, slot * sq, cell_off);
+        }
+    }
+};
 
 // Element offset of cell (x, y, z) (interior coordinates), periodic axes wrapped; false when the
 // cell lies beyond the ghost layer of a non-periodic axis.  Used by the boundary conditions that
@@ -113,7 +149,7 @@ __device__ __forceinline__ R load_f_out(const SweepArgs& a, int x, int y, int z,
     if (!cell_offset(a.g, x + ox + PA::template woff<Q>(d, 0), y + oy + PA::template woff<Q>(d, 1),
                      z + oz + PA::template woff<Q>(d, 2), off))
         return fallback;
-    return Conv<S, R>::ld(static_cast<const S*>(a.src) + eidx(PA::template wslot<Q>(d) * a.g.sq, off));
+    return Conv<S, R>::ld(at(static_cast<const S*>(a.src), PA::template wslot<Q>(d) * a.g.sq, off));
 }
 
 // Fused boundary handling for a fluid cell next to a boundary: replaces the pulled value of every
@@ -130,7 +166,7 @@ __device__ __forceinline__ R load_f_out(const SweepArgs& a, int x, int y, int z,
 // ends every warp of a cavity has one.  The directions come as one word per cell (`w`, wall_word), so
 // the bounced populations are fetched together after a single load, where a flag per neighbour cost
 // up to Q - 1 dependent round trips, one after another.
-template <class S, class R, int Q, int PAT>
+template <class S, class R, int Q, int PAT, bool SHARED_ARGS = false>
 __device__ __forceinline__ void bounce_back(R (&f)[Q], const SweepArgs& a, const NbrOffsets& nb, int cell,
                                          int x, int y, int z, uint32_t w) {
     using L = Lat<Q>;
@@ -139,13 +175,15 @@ __device__ __forceinline__ void bounce_back(R (&f)[Q], const SweepArgs& a, const
     const S* src = static_cast<const S*>(a.src);
     // Interior cell indices fit 32 bits (the host bounds the field below 2^32 elements).
     const unsigned icell = unsigned(x) + unsigned(g.nx) * (unsigned(y) + unsigned(g.ny) * unsigned(z));
+    Slots<const S, SHARED_ARGS> slots(src, g.sq);
 #pragma unroll
-    for (int i = 1; i < Q; ++i) {
-        if (!((w >> i) & 1u)) continue;
-        // f_out(x, inv i): where the previous step wrote direction inv(i) of this cell
-        const int j = L::inv(i);
+    for (int s = 0; s < Q; ++s) {
+        // slot s holds f_out(x, j), which replaces direction i = inv(j): where the previous step
+        // wrote direction j of this cell (its slot rule is its own inverse)
+        const int j = PA::template wslot<Q>(s), i = L::inv(j);
         const int off = nb.off(PA::template woff<Q>(j, 0), PA::template woff<Q>(j, 1), PA::template woff<Q>(j, 2));
-        f[i] = Conv<S, R>::ld(src + eidx(PA::template wslot<Q>(j) * g.sq, cell + off));
+        const S* q = slots(s, cell + off);
+        if (i > 0 && ((w >> i) & 1u)) f[i] = Conv<S, R>::ld(q);
     }
     if (!(w & WALL_UBB)) return;
     const uint32_t um = g.walls != nullptr ? g.walls[size_t(g.wall_plane) + icell] : (w | WALL_UBB_MIXED);
@@ -190,7 +228,7 @@ __device__ __forceinline__ void bounce_back(R (&f)[Q], const SweepArgs& a, const
 
 // The whole update of one cell: pull through the accessor, fused bounce-back, collision, push
 // through the accessor.  Shared by the single-domain and the batched sweeps.
-template <class S, class R, int Q, int MK, int PAT>
+template <class S, class R, int Q, int MK, int PAT, bool SHARED_ARGS = false>
 __device__ __forceinline__ void sweep_cell(const SweepArgs& a, int x, int y, int z) {
     using A = Access<PAT>;
     const Grid& g = a.g;
@@ -208,18 +246,22 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs& a, int x, int y, int
     const S* src = static_cast<const S*>(a.src);
     S* dst = static_cast<S*>(a.dst);
     R f[Q];
+    Slots<const S, SHARED_ARGS> rs(src, g.sq);
 #pragma unroll
-    for (int i = 0; i < Q; ++i) {
+    for (int s = 0; s < Q; ++s) {
+        const int i = A::template rslot<Q>(s);       // the slot rule is its own inverse
         const int off = nb.off(A::template roff<Q>(i, 0), A::template roff<Q>(i, 1), A::template roff<Q>(i, 2));
-        f[i] = Conv<S, R>::ld(src + eidx(A::template rslot<Q>(i) * g.sq, cell + off));
+        f[i] = Conv<S, R>::ld(rs(s, cell + off));
     }
     if (!word_first && (w & WALL_SELF)) return;
-    if (w != 0) bounce_back<S, R, Q, PAT>(f, a, nb, cell, x, y, z, w);
+    if (w != 0) bounce_back<S, R, Q, PAT, SHARED_ARGS>(f, a, nb, cell, x, y, z, w);
     const R om = collide<R, Q, MK>(f, a.p);
+    Slots<S, SHARED_ARGS> ws(dst, g.sq);
 #pragma unroll
-    for (int i = 0; i < Q; ++i) {
+    for (int s = 0; s < Q; ++s) {
+        const int i = A::template wslot<Q>(s);
         const int off = nb.off(A::template woff<Q>(i, 0), A::template woff<Q>(i, 1), A::template woff<Q>(i, 2));
-        Conv<S, R>::st(dst + eidx(A::template wslot<Q>(i) * g.sq, cell + off), f[i]);
+        Conv<S, R>::st(ws(s, cell + off), f[i]);
     }
     if (a.omega_out != nullptr) a.omega_out[x + g.nx * (y + (long long)g.ny * z)] = (float)om;
 }
@@ -231,12 +273,12 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs& a, int x, int y, int
 // of the copy bandwidth; 0.92 at 64).  These hot variants are held to register counts checked
 // for spills with -Xptxas -v: 80 (3 blocks), 64 (4) and 48 (5).
 template <class S, int Q, int MK, int PAT> struct SweepMinBlocks { static constexpr int value = 1; };
-template <> struct SweepMinBlocks<float, 27, MK_CUM1, PAT_AA_ODD> { static constexpr int value = 3; };
+template <> struct SweepMinBlocks<float, 27, MK_CUM1, PAT_AA_ODD> { static constexpr int value = 4; };
 template <> struct SweepMinBlocks<float, 27, MK_CUM1, PAT_AA_EVEN> { static constexpr int value = 4; };
 template <> struct SweepMinBlocks<float, 19, MK_POP, PAT_PULL> { static constexpr int value = 5; };
 template <> struct SweepMinBlocks<float, 19, MK_POP, PAT_AA_ODD> { static constexpr int value = 4; };
 template <> struct SweepMinBlocks<float, 19, MK_POP, PAT_AA_EVEN> { static constexpr int value = 4; };
-template <> struct SweepMinBlocks<float, 27, MK_POP, PAT_AA_ODD> { static constexpr int value = 3; };
+template <> struct SweepMinBlocks<float, 27, MK_POP, PAT_AA_ODD> { static constexpr int value = 4; };
 template <> struct SweepMinBlocks<float, 27, MK_POP, PAT_AA_EVEN> { static constexpr int value = 4; };
 template <> struct SweepMinBlocks<float, 19, MK_MRT, PAT_PULL> { static constexpr int value = 4; };
 template <> struct SweepMinBlocks<float, 27, MK_MRT, PAT_PULL> { static constexpr int value = 3; };
@@ -275,7 +317,7 @@ __global__ void __launch_bounds__(256, 2) k_sweep_zpipe(const SweepArgs a) {
 #pragma unroll
         for (int i = 0; i < Q; ++i) {
             const int off = nb.off(A::template roff<Q>(i, 0), A::template roff<Q>(i, 1), A::template roff<Q>(i, 2));
-            h[i] = Conv<S, R>::ld(src + eidx(A::template rslot<Q>(i) * g.sq, cell + off));
+            h[i] = Conv<S, R>::ld(at(src, A::template rslot<Q>(i) * g.sq, cell + off));
         }
     };
     R nxt[Q];
@@ -297,7 +339,7 @@ __global__ void __launch_bounds__(256, 2) k_sweep_zpipe(const SweepArgs a) {
 #pragma unroll
         for (int i = 0; i < Q; ++i) {
             const int off = nb.off(A::template woff<Q>(i, 0), A::template woff<Q>(i, 1), A::template woff<Q>(i, 2));
-            Conv<S, R>::st(dst + eidx(A::template wslot<Q>(i) * g.sq, cell + off), f[i]);
+            Conv<S, R>::st(at(dst, A::template wslot<Q>(i) * g.sq, cell + off), f[i]);
         }
     }
 }
@@ -315,7 +357,7 @@ __device__ __forceinline__ void prefetch_cell(const SweepArgs& a, int x, int y, 
 #pragma unroll
     for (int i = 0; i < Q; ++i) {
         const int off = nb.off(A::template roff<Q>(i, 0), A::template roff<Q>(i, 1), A::template roff<Q>(i, 2));
-        const S* q = src + eidx(A::template rslot<Q>(i) * g.sq, cell + off);
+        const S* q = at(src, A::template rslot<Q>(i) * g.sq, cell + off);
         asm volatile("prefetch.global.L2 [%0];" ::"l"(q));
     }
 }
@@ -344,7 +386,7 @@ __global__ void __launch_bounds__(256) k_ubb_density(const SweepArgs a, R* rho_o
 #pragma unroll
     for (int k = 0; k < Q; ++k) {
         const int ok = nb.off(PA::template woff<Q>(k, 0), PA::template woff<Q>(k, 1), PA::template woff<Q>(k, 2));
-        s += Conv<S, R>::ld(src + eidx(PA::template wslot<Q>(k) * g.sq, cell + ok));
+        s += Conv<S, R>::ld(at(src, PA::template wslot<Q>(k) * g.sq, cell + ok));
     }
     rho_out[x + g.nx * (y + g.ny * z)] = R(1) + s;
 }
@@ -368,8 +410,11 @@ struct BatchArgs {
     int parity;                   // selects which half of `domains` (src/dst swapped) to use
 };
 
+// Resident 256-thread blocks per SM that the batched sweep is compiled for.
+template <class S, int Q, int MK> struct BatchMinBlocks { static constexpr int value = 3; };
+
 template <class S, class R, int Q, int MK, int PAT>
-__global__ void __launch_bounds__(256, 3) k_sweep_batched(const BatchArgs b) {
+__global__ void __launch_bounds__(256, BatchMinBlocks<S, Q, MK>::value) k_sweep_batched(const BatchArgs b) {
     __shared__ __align__(16) SweepArgs sa;
     constexpr int WORDS = sizeof(SweepArgs) / 4;
     static_assert(sizeof(SweepArgs) % 4 == 0, "SweepArgs is copied as 32-bit words");
@@ -392,7 +437,7 @@ __global__ void __launch_bounds__(256, 3) k_sweep_batched(const BatchArgs b) {
         if (x < sa.g.nx && y < sa.g.ny) {
             const int z1 = min(tile.z0 + b.cells_z, sa.g.nz);
 #pragma unroll 1
-            for (int z = tile.z0; z < z1; ++z) sweep_cell<S, R, Q, MK, PAT>(sa, x, y, z);
+            for (int z = tile.z0; z < z1; ++z) sweep_cell<S, R, Q, MK, PAT, true>(sa, x, y, z);
         }
     }
 }
@@ -404,7 +449,7 @@ __global__ void __launch_bounds__(256, 3) k_sweep_batched(const BatchArgs b) {
 // (a neighbour's slot, the cell's own inverse slot for NoSlip, or the periodic image).  Index
 // layout here: [Q-1][n_fluid] (direction-major, so a warp's reads of one direction are coalesced).
 struct SparseArgs {
-    Physics p;
+    SweepPhysics p;
     const void* src;
     void* dst;
     const unsigned* index;
@@ -535,7 +580,7 @@ __global__ void __launch_bounds__(256) k_set_equilibrium(const MacroArgs a) {
 #pragma unroll
     for (int i = 0; i < Q; ++i) {
         const int off = nb.off(A::template woff<Q>(i, 0), A::template woff<Q>(i, 1), A::template woff<Q>(i, 2));
-        Conv<S, R>::st(dst + eidx(A::template wslot<Q>(i) * g.sq, cell + off), f[i]);
+        Conv<S, R>::st(at(dst, A::template wslot<Q>(i) * g.sq, cell + off), f[i]);
     }
 }
 
@@ -597,12 +642,12 @@ __global__ void __launch_bounds__(256) k_boundary_prepass(const SweepArgs a) {
 #pragma unroll
     for (int k = 0; k < Q; ++k) {
         const int off = nb.off(PA::template woff<Q>(k, 0), PA::template woff<Q>(k, 1), PA::template woff<Q>(k, 2));
-        out[k] = Conv<S, R>::ld(f + eidx(PA::template wslot<Q>(k) * g.sq, cell + off));
+        out[k] = Conv<S, R>::ld(at(f, PA::template wslot<Q>(k) * g.sq, cell + off));
     }
     // where the sweep reads direction i of this cell
     auto store = [&](int i, R v) {
         const int off = nb.off(A::template roff<Q>(i, 0), A::template roff<Q>(i, 1), A::template roff<Q>(i, 2));
-        Conv<S, R>::st(f + eidx(A::template rslot<Q>(i) * g.sq, cell + off), v);
+        Conv<S, R>::st(at(f, A::template rslot<Q>(i) * g.sq, cell + off), v);
     };
     if (types & ((1u << FLAG_FIXED_DENSITY) | (1u << FLAG_FIXED_DENSITY1))) {
         R jx = 0, jy = 0, jz = 0;
@@ -684,7 +729,7 @@ __global__ void __launch_bounds__(256) k_get_macroscopic(const MacroArgs a) {
 #pragma unroll
     for (int i = 0; i < Q; ++i) {
         const int off = nb.off(A::template woff<Q>(i, 0), A::template woff<Q>(i, 1), A::template woff<Q>(i, 2));
-        f[i] = Conv<S, R>::ld(src + eidx(A::template wslot<Q>(i) * g.sq, cell + off));
+        f[i] = Conv<S, R>::ld(at(src, A::template wslot<Q>(i) * g.sq, cell + off));
     }
     Macro<Q, R> m = conserved<Q, R>(f, a.p, false);
     if (a.p.force_model != FM_NONE) {

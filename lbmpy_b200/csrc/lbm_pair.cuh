@@ -76,13 +76,8 @@ template <> struct Pair<__nv_bfloat16> {
     __device__ __forceinline__ static V from_f2(float2 v) { return __float22bfloat162_rn(v); }
 };
 
-template <class R, int Q, int MK>
-__device__ __forceinline__ F2 collide2(F2 (&f)[Q], const Physics& p) {
-    if constexpr (MK == MK_POP) return collide_pop<Q, F2>(f, p);
-    else if constexpr (MK == MK_MRT) return collide_mrt<Q, F2>(f, p);
-    else if constexpr (MK == MK_CUM1) return collide_cum_ho1<F2>(f, p);
-    else return collide_cum<F2>(f, p);
-}
+template <class R, int Q, int MK, class P>
+__device__ __forceinline__ F2 collide2(F2 (&f)[Q], const P& p) { return Collision<MK>::template run<Q, F2>(f, p); }
 
 // One warp covers 32 pairs = 64 cells of one x row; block = 32 x PAIR_ROWS threads.
 constexpr int PAIR_ROWS = 4;
@@ -140,17 +135,17 @@ __global__ void __launch_bounds__(32 * PAIR_ROWS, PairMinBlocks<S>::value) k_swe
         const int yz = nbA.off(0, A::template roff<Q>(i, 1), A::template roff<Q>(i, 2));
         const unsigned slot = A::template rslot<Q>(i) * g.sq;
         // aligned pair of the source row at (x0, x0 + 1)
-        const float2 P = PS::to_f2(PS::ld(src + eidx(slot, cellA + yz)));
+        const float2 P = PS::to_f2(PS::ld(at(src, slot, cellA + yz)));
         float va, vb;
         if (cx == 0) {
             va = P.x; vb = P.y;
         } else if (cx == -1) {                     // cells read x - 1: (x0 - 1, x0)
             float up = __shfl_up_sync(0xffffffffu, P.y, 1);
-            if (lane == 0) up = Conv<S, float>::ld(src + eidx(slot, cellA + yz + nbA.dx[0]));
+            if (lane == 0) up = Conv<S, float>::ld(at(src, slot, cellA + yz + nbA.dx[0]));
             va = up; vb = P.x;
         } else {                                   // cells read x + 1: (x0 + 1, x0 + 2)
             float dn = __shfl_down_sync(0xffffffffu, P.x, 1);
-            if (lane == last_lane) dn = Conv<S, float>::ld(src + eidx(slot, cellA + 1 + yz + nbB.dx[2]));
+            if (lane == last_lane) dn = Conv<S, float>::ld(at(src, slot, cellA + 1 + yz + nbB.dx[2]));
             va = P.y; vb = dn;
         }
         f[i] = F2(va, vb);
@@ -173,7 +168,7 @@ __global__ void __launch_bounds__(32 * PAIR_ROWS, PairMinBlocks<S>::value) k_swe
         const bool keepA = (wA & WALL_SELF) != 0, keepB = (wB & WALL_SELF) != 0;
 #pragma unroll
         for (int i = 0; i < Q; ++i) {
-            const S* q = src + eidx(L::inv(i) * g.sq, cellA);
+            const S* q = at(src, L::inv(i) * g.sq, cellA);
             f[i] = F2(keepA ? Conv<S, float>::ld(q) : f[i].v.x, keepB ? Conv<S, float>::ld(q + 1) : f[i].v.y);
         }
     }
@@ -185,20 +180,20 @@ __global__ void __launch_bounds__(32 * PAIR_ROWS, PairMinBlocks<S>::value) k_swe
         const unsigned slot = A::template wslot<Q>(i) * g.sq;
         const float va = f[i].v.x, vb = f[i].v.y;
         if (cx == 0) {
-            if (active) PS::st(dst + eidx(slot, cellA + yz), PS::from_f2(make_float2(va, vb)));
+            if (active) PS::st(at(dst, slot, cellA + yz), PS::from_f2(make_float2(va, vb)));
         } else if (cx == 1) {                      // A -> x0 + 1, B -> x0 + 2
             const float prevB = __shfl_up_sync(0xffffffffu, vb, 1);
             if (active) {
-                if (lane == 0) Conv<S, float>::st(dst + eidx(slot, cellA + 1 + yz), va);
-                else PS::st(dst + eidx(slot, cellA + yz), PS::from_f2(make_float2(prevB, va)));
-                if (lane == last_lane) Conv<S, float>::st(dst + eidx(slot, cellA + 1 + yz + nbB.dx[2]), vb);
+                if (lane == 0) Conv<S, float>::st(at(dst, slot, cellA + 1 + yz), va);
+                else PS::st(at(dst, slot, cellA + yz), PS::from_f2(make_float2(prevB, va)));
+                if (lane == last_lane) Conv<S, float>::st(at(dst, slot, cellA + 1 + yz + nbB.dx[2]), vb);
             }
         } else {                                   // A -> x0 - 1, B -> x0
             const float nextA = __shfl_down_sync(0xffffffffu, va, 1);
             if (active) {
-                if (lane == last_lane) Conv<S, float>::st(dst + eidx(slot, cellA + yz), vb);
-                else PS::st(dst + eidx(slot, cellA + yz), PS::from_f2(make_float2(vb, nextA)));
-                if (lane == 0) Conv<S, float>::st(dst + eidx(slot, cellA + yz + nbA.dx[0]), va);
+                if (lane == last_lane) Conv<S, float>::st(at(dst, slot, cellA + yz), vb);
+                else PS::st(at(dst, slot, cellA + yz), PS::from_f2(make_float2(vb, nextA)));
+                if (lane == 0) Conv<S, float>::st(at(dst, slot, cellA + yz + nbA.dx[0]), va);
             }
         }
     }

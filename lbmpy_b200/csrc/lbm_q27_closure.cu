@@ -73,7 +73,7 @@ __global__ void __launch_bounds__(256, 3) k_sweep_closure_tc(const SweepArgs a) 
 #pragma unroll
         for (int i = 0; i < 27; ++i) {
             const int off = nb.off(A::template roff<27>(i, 0), A::template roff<27>(i, 1), A::template roff<27>(i, 2));
-            f[i] = src[eidx(A::template rslot<27>(i) * g.sq, cell + off)];
+            f[i] = *at(src, A::template rslot<27>(i) * g.sq, cell + off);
         }
         const bool fluid = inside && !(w & WALL_SELF);
         if (fluid && w != 0) bounce_back<float, float, 27, PAT>(f, a, nb, cell, x, y, z, w);
@@ -83,7 +83,7 @@ __global__ void __launch_bounds__(256, 3) k_sweep_closure_tc(const SweepArgs a) 
 #pragma unroll
             for (int i = 0; i < 27; ++i) {
                 const int off = nb.off(A::template woff<27>(i, 0), A::template woff<27>(i, 1), A::template woff<27>(i, 2));
-                dst[eidx(A::template wslot<27>(i) * g.sq, cell + off)] = f[i];
+                *at(dst, A::template wslot<27>(i) * g.sq, cell + off) = f[i];
             }
             if (a.omega_out != nullptr) a.omega_out[x + g.nx * (y + (long long)g.ny * z)] = om;
         }

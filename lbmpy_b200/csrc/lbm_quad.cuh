@@ -90,17 +90,17 @@ __global__ void __launch_bounds__(32 * QUAD_ROWS, 4) k_sweep_quad(const SweepArg
         const int yz = nbA.off(0, A::template roff<Q>(i, 1), A::template roff<Q>(i, 2));
         const unsigned slot = A::template rslot<Q>(i) * g.sq;
         float P[4];
-        quad_ld<S>(src + eidx(slot, cellA + yz), P);
+        quad_ld<S>(at(src, slot, cellA + yz), P);
         float v[4];
         if (cx == 0) {
             v[0] = P[0]; v[1] = P[1]; v[2] = P[2]; v[3] = P[3];
         } else if (cx == -1) {                     // cells read x - 1: (x0 - 1 .. x0 + 2)
             float up = __shfl_up_sync(0xffffffffu, P[3], 1);
-            if (lane == 0) up = Conv<S, float>::ld(src + eidx(slot, cellA + yz + nbA.dx[0]));
+            if (lane == 0) up = Conv<S, float>::ld(at(src, slot, cellA + yz + nbA.dx[0]));
             v[0] = up; v[1] = P[0]; v[2] = P[1]; v[3] = P[2];
         } else {                                   // cells read x + 1: (x0 + 1 .. x0 + 4)
             float dn = __shfl_down_sync(0xffffffffu, P[0], 1);
-            if (lane == last_lane) dn = Conv<S, float>::ld(src + eidx(slot, cellA + 3 + yz + nbD.dx[2]));
+            if (lane == last_lane) dn = Conv<S, float>::ld(at(src, slot, cellA + 3 + yz + nbD.dx[2]));
             v[0] = P[1]; v[1] = P[2]; v[2] = P[3]; v[3] = dn;
         }
         f0[i] = F2(v[0], v[1]);
@@ -134,7 +134,7 @@ __global__ void __launch_bounds__(32 * QUAD_ROWS, 4) k_sweep_quad(const SweepArg
     if (PAT == PAT_AA_EVEN && ((w[0] | w[1] | w[2] | w[3]) & WALL_SELF)) {
 #pragma unroll
         for (int i = 0; i < Q; ++i) {
-            const S* q = src + eidx(L::inv(i) * g.sq, cellA);
+            const S* q = at(src, L::inv(i) * g.sq, cellA);
             if (w[0] & WALL_SELF) f0[i].v.x = Conv<S, float>::ld(q);
             if (w[1] & WALL_SELF) f0[i].v.y = Conv<S, float>::ld(q + 1);
             if (w[2] & WALL_SELF) f1[i].v.x = Conv<S, float>::ld(q + 2);
@@ -149,32 +149,32 @@ __global__ void __launch_bounds__(32 * QUAD_ROWS, 4) k_sweep_quad(const SweepArg
         const unsigned slot = A::template wslot<Q>(i) * g.sq;
         const float va = f0[i].v.x, vb = f0[i].v.y, vc = f1[i].v.x, vd = f1[i].v.y;
         if (cx == 0) {
-            if (active) quad_st<S>(dst + eidx(slot, cellA + yz), va, vb, vc, vd);
+            if (active) quad_st<S>(at(dst, slot, cellA + yz), va, vb, vc, vd);
         } else if (cx == 1) {                      // A..D -> x0+1 .. x0+4
             const float prevD = __shfl_up_sync(0xffffffffu, vd, 1);
             if (active) {
                 if (lane == 0) {                   // x0 belongs to the previous warp's last lane
-                    S* p = dst + eidx(slot, cellA + yz);
+                    S* p = at(dst, slot, cellA + yz);
                     Conv<S, float>::st(p + 1, va);
                     Conv<S, float>::st(p + 2, vb);
                     Conv<S, float>::st(p + 3, vc);
                 } else {
-                    quad_st<S>(dst + eidx(slot, cellA + yz), prevD, va, vb, vc);
+                    quad_st<S>(at(dst, slot, cellA + yz), prevD, va, vb, vc);
                 }
-                if (lane == last_lane) Conv<S, float>::st(dst + eidx(slot, cellA + 3 + yz + nbD.dx[2]), vd);
+                if (lane == last_lane) Conv<S, float>::st(at(dst, slot, cellA + 3 + yz + nbD.dx[2]), vd);
             }
         } else {                                   // A..D -> x0-1 .. x0+2
             const float nextA = __shfl_down_sync(0xffffffffu, va, 1);
             if (active) {
                 if (lane == last_lane) {           // x0+3 belongs to the next warp's lane 0
-                    S* p = dst + eidx(slot, cellA + yz);
+                    S* p = at(dst, slot, cellA + yz);
                     Conv<S, float>::st(p, vb);
                     Conv<S, float>::st(p + 1, vc);
                     Conv<S, float>::st(p + 2, vd);
                 } else {
-                    quad_st<S>(dst + eidx(slot, cellA + yz), vb, vc, vd, nextA);
+                    quad_st<S>(at(dst, slot, cellA + yz), vb, vc, vd, nextA);
                 }
-                if (lane == 0) Conv<S, float>::st(dst + eidx(slot, cellA + yz + nbA.dx[0]), va);
+                if (lane == 0) Conv<S, float>::st(at(dst, slot, cellA + yz + nbA.dx[0]), va);
             }
         }
     }

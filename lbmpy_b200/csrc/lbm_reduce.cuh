@@ -29,7 +29,7 @@ __global__ void __launch_bounds__(RED_THREADS) k_reduce_partial(const MacroArgs 
 #pragma unroll
         for (int i = 0; i < Q; ++i) {
             const int off = nb.off(A::template woff<Q>(i, 0), A::template woff<Q>(i, 1), A::template woff<Q>(i, 2));
-            f[i] = Conv<S, double>::ld(src + eidx(A::template wslot<Q>(i) * g.sq, cell + off));
+            f[i] = Conv<S, double>::ld(at(src, A::template wslot<Q>(i) * g.sq, cell + off));
         }
         Macro<Q, double> m = conserved<Q, double>(f, a.p, false);
         if (a.p.force_model != FM_NONE) {

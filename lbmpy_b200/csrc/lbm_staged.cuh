@@ -194,7 +194,7 @@ __global__ void __launch_bounds__(W) k_sweep_staged(const SweepArgs a, const int
             constexpr int WP = decltype(wp)::value;
 #pragma unroll
             for (int i = WP; i < Q; i += NW) {
-                const S* row = src + eidx(A::template rslot<Q>(i) * g.sq,
+                const S* row = at(src, A::template rslot<Q>(i) * g.sq,
                                           cell + nb.off(0, A::template roff<Q>(i, 1), A::template roff<Q>(i, 2)));
                 const char* rowb = reinterpret_cast<const char*>(row);
                 S* sr = st + i * Lay::PS + Lay::PADE;
@@ -273,7 +273,7 @@ __global__ void __launch_bounds__(W) k_sweep_staged(const SweepArgs a, const int
 #pragma unroll
             for (int i = 0; i < Q; ++i) {
                 const int off = nb.off(A::template woff<Q>(i, 0), A::template woff<Q>(i, 1), A::template woff<Q>(i, 2));
-                Conv<S, R>::st(dst + eidx(A::template wslot<Q>(i) * g.sq, cell + off), f[i]);
+                Conv<S, R>::st(at(dst, A::template wslot<Q>(i) * g.sq, cell + off), f[i]);
             }
             if (a.omega_out != nullptr) a.omega_out[x + g.nx * (t.y + (long long)g.ny * t.z)] = (float)om;
         }
