@@ -33,10 +33,9 @@ struct LbmPlan {
     int block_x;           // x extent of the one-cell sweep's 256-thread blocks, 0 automatic (LBM_B200_BX)
     int sms;               // multiprocessors of the plan's device
     unsigned* status;      // device status word (lbm_plan_status), inside the reduction scratch
-    uint32_t* rowmask;     // row summary of the flag field last finalized with this plan
+    mutable uint32_t* rowmask;             // row summary of the flag field last finalized with this plan
     mutable const uint8_t* rowmask_flags;  // that flag field (sweeps given it use the summary)
-    mutable uint32_t* walls;               // wall words of that flag field (three planes), or nullptr
-    mutable bool walls_valid;              // they belong to rowmask_flags
+    mutable uint32_t* walls;               // its wall words, behind the row summary
     void* ubb_rho;         // compressible + moving UBB walls: density gathered before the sweep
     const int* ubb_block;  // per-link boundary tables (lbm_plan_set_links), caller-owned
     const double* ubb_link_vel;
@@ -127,7 +126,6 @@ Grid make_grid(const LbmPlan* p, const int64_t s[4], const uint8_t* flags) {
     g.fsz = (g.nx + 2) * (g.ny + 2);
     g.rowmask = nullptr;
     g.walls = nullptr;
-    g.wall_plane = unsigned(g.nx) * unsigned(g.ny) * unsigned(g.nz);
     return g;
 }
 
@@ -220,12 +218,13 @@ bool quad_applicable(const LbmPlan* p, const void* src, const void* dst, const i
 // The pair sweep needs an even row length, no omega output, and every row's interior cell x = 0
 // (ghost-inclusive x = 1) on a 2-element boundary so that paired loads / stores are aligned.
 // Default policy, from B200 measurements: the pair sweep wins where the one-cell sweep is limited by
-// instruction issue (16-bit storage, the cumulant with pull streaming); for FP32 storage the
-// one-cell sweep already streams at HBM speed and keeps twice the occupancy.
+// instruction issue: 16-bit storage, and the general cumulant with pull streaming.  The specialised
+// cumulant's one-cell sweep holds 64 registers (4 blocks per SM) and has caught up with it (pull FP32
+// 256x128x128: channel 158 us, periodic 155 us; pair 161 us periodic at 96 registers).
 bool pair_preferred(const LbmPlan* p, int pat) {
     if (p->use_pair >= 0) return p->use_pair == 1;
     if (p->store == ST_F16 || p->store == ST_BF16 || p->store == ST_E3M12) return true;
-    return (p->mk == MK_CUM || p->mk == MK_CUM1) && pat == PAT_PULL;
+    return p->mk == MK_CUM && pat == PAT_PULL;
 }
 
 bool pair_applicable(const LbmPlan* p, const void* src, const void* dst, const int64_t s[4], int pat,
@@ -479,8 +478,7 @@ __global__ void k_flags_finalize(Grid g) {
     fl[fc] = (uint8_t)v;
 }
 
-// Wall words of a finalized flag field (WALL_* in lbm_common.cuh): three planes of one word per
-// interior cell.
+// Wall words of a finalized flag field (WALL_* in lbm_common.cuh), one per interior cell.
 template <int Q>
 __global__ void __launch_bounds__(256) k_wall_words(Grid g, uint32_t* words) {
     using L = Lat<Q>;
@@ -490,36 +488,23 @@ __global__ void __launch_bounds__(256) k_wall_words(Grid g, uint32_t* words) {
     if (x >= g.nx || y >= g.ny) return;
     const uint8_t* cell = g.flags + ((x + 1) + (y + 1) * g.fsy + (z + 1) * g.fsz);
     const int fl = *cell;
-    uint32_t w = 0, ubb = 0, per_link = 0;
+    uint32_t w = 0;
     if (fl & FLAG_TYPE_MASK) {
         w = WALL_SELF;
     } else if (fl & FLAG_NEAR_WALL) {
-        NbrOffsets fo;
-        Grid gf = g;
-        gf.sy = g.fsy;
-        gf.sz = g.fsz;
-        fo.init(gf, x, y, z);
+        const NbrOffsets fo = flag_offsets(g, x, y, z);
         unsigned types = 0;   // bit t: a link to a cell of type t
 #pragma unroll
         for (int i = 1; i < Q; ++i) {
             const int t = cell[fo.off(-L::cx(i), -L::cy(i), -L::cz(i))] & FLAG_TYPE_MASK;
             types |= 1u << t;
             if (t == FLAG_NOSLIP || flag_is_ubb(t)) w |= 1u << i;
-            if (flag_is_ubb(t)) ubb |= 1u << i;
-            if (t >= FLAG_FREE_SLIP) per_link |= 1u << i;
         }
         if (types & ((1u << FLAG_FIXED_DENSITY) | (1u << FLAG_FIXED_DENSITY1))) w |= WALL_FIXED_DENSITY;
-        if (per_link) w |= WALL_PER_LINK;
-        if (ubb) {
-            w |= WALL_UBB;
-            const unsigned numbers = (types >> FLAG_UBB0) & ((1u << MAX_UBB) - 1u);
-            ubb |= (numbers & (numbers - 1u)) ? WALL_UBB_MIXED : uint32_t(__ffs(int(numbers)) - 1) << WALL_UBB_SHIFT;
-        }
+        if (types >> FLAG_FREE_SLIP) w |= WALL_PER_LINK;
+        if ((types >> FLAG_UBB0) & ((1u << MAX_UBB) - 1u)) w |= WALL_UBB;
     }
-    const size_t c = size_t(x) + size_t(g.nx) * (size_t(y) + size_t(g.ny) * z);
-    words[c] = w;
-    words[c + g.wall_plane] = ubb;
-    words[c + 2 * size_t(g.wall_plane)] = per_link;
+    words[size_t(x) + size_t(g.nx) * (size_t(y) + size_t(g.ny) * z)] = w;
 }
 
 cudaError_t launch_wall_words(int q, const Grid& g, uint32_t* words, cudaStream_t s) {
@@ -750,7 +735,6 @@ int lbm_plan_create(const LbmPlanDesc* desc, LbmPlan** out) {
     p->rowmask = nullptr;
     p->rowmask_flags = nullptr;
     p->walls = nullptr;
-    p->walls_valid = false;
     if (sweep_launcher(p, PAT_PULL) == nullptr) {
         cudaFree(p->partial);
         delete p;
@@ -760,13 +744,6 @@ int lbm_plan_create(const LbmPlanDesc* desc, LbmPlan** out) {
         cudaFree(p->partial);
         delete p;
         return rc2;
-    }
-    e = cudaMalloc(&p->rowmask, rowmask_bytes(p));
-    if (e != cudaSuccess) {
-        cudaFree(p->partial);
-        if (p->ubb_rho) cudaFree(p->ubb_rho);
-        delete p;
-        return cuda_fail(e, "cudaMalloc(row summary)");
     }
     *out = p;
     return LBM_OK;
@@ -791,7 +768,6 @@ int lbm_plan_destroy(LbmPlan* p) {
     if (p->partial) cudaFree(p->partial);
     if (p->ubb_rho) cudaFree(p->ubb_rho);
     if (p->rowmask) cudaFree(p->rowmask);
-    if (p->walls) cudaFree(p->walls);
     delete p;
     return LBM_OK;
 }
@@ -848,7 +824,7 @@ static int launch_sweep_checked(const LbmPlan* p, const void* src, void* dst, co
     a.link_value = p->link_value;
     if (flags != nullptr && flags == p->rowmask_flags) {
         a.g.rowmask = p->rowmask;
-        if (p->walls_valid) a.g.walls = p->walls;
+        a.g.walls = p->walls;
     }
     if (flags != nullptr && p->ubb_rho != nullptr && needs_ubb_density(&p->desc, p->ubb_link_mask)) {
         UbbLauncher U = p->q == 19 ? ubb_launcher_q<19>(p->store, pat) : ubb_launcher_q<27>(p->store, pat);
@@ -1059,29 +1035,28 @@ int lbm_flags_finalize(const LbmPlan* p, uint8_t* flags, void* stream) {
     else k_flags_finalize<27><<<grid, block, 0, st>>>(g);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(e, "flag finalize launch");
-    // the row summary the sweeps of this plan use with this flag field
+    // The row summary and the wall words the sweeps of this plan use with this flag field.  Without the
+    // memory for them (or while a graph is being captured, when it cannot be allocated) the sweeps
+    // take the walls from the flags.
     p->rowmask_flags = nullptr;
-    p->walls_valid = false;
-    e = cudaMemsetAsync(p->rowmask, 0, rowmask_bytes(p), st);
+    const size_t rows = rowmask_bytes(p), cells = size_t(g.nx) * g.ny * g.nz;
+    if (p->rowmask == nullptr) {
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(st, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone ||
+            cudaMalloc(&p->rowmask, rows + sizeof(uint32_t) * cells) != cudaSuccess) {
+            p->rowmask = nullptr;
+            cudaGetLastError();
+            return LBM_OK;
+        }
+        p->walls = p->rowmask + rows / sizeof(uint32_t);
+    }
+    e = cudaMemsetAsync(p->rowmask, 0, rows, st);
     if (e != cudaSuccess) return cuda_fail(e, "clearing the row summary");
-    const int rows = g.ny * g.nz;
-    k_row_mask<<<(rows + 255) / 256, 256, 0, st>>>(g, p->rowmask);
+    k_row_mask<<<(g.ny * g.nz + 255) / 256, 256, 0, st>>>(g, p->rowmask);
     e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(e, "row summary launch");
-    // and their wall words; without the memory for them (or while a graph is being captured, when it
-    // cannot be allocated) the sweeps take the walls from the flags
-    if (p->walls == nullptr) {
-        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-        if (cudaStreamIsCapturing(st, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone &&
-            cudaMalloc(&p->walls, 3 * sizeof(uint32_t) * size_t(g.wall_plane)) != cudaSuccess)
-            p->walls = nullptr;
-        cudaGetLastError();
-    }
-    if (p->walls != nullptr) {
-        e = launch_wall_words(p->q, g, p->walls, st);
-        if (e != cudaSuccess) return cuda_fail(e, "wall word launch");
-        p->walls_valid = true;
-    }
+    e = launch_wall_words(p->q, g, p->walls, st);
+    if (e != cudaSuccess) return cuda_fail(e, "wall word launch");
     p->rowmask_flags = flags;
     return LBM_OK;
 }
@@ -1157,7 +1132,7 @@ cudaError_t launch_sparse_get(const SparseArgs& a, double* rho, double* u, cudaS
 template <class S, class R, int Q>
 cudaError_t launch_sparse_ubb(const SparseArgs& a, const uint32_t* links, int64_t n, const double* u,
                               cudaStream_t s) {
-    k_sparse_ubb<S, R, Q><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(a, links, n, u[0], u[1], u[2]);
+    k_sparse_ubb<S, R, Q><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(a, links, (long long)n, u[0], u[1], u[2]);
     return cudaGetLastError();
 }
 
@@ -1448,13 +1423,13 @@ int lbm_batch_create(const LbmPlanDesc* common, const LbmDomainDesc* domains, in
     b->d_walls = nullptr;
     size_t wall_words = 0;
     for (int k = 0; k < n_domains; ++k)
-        if (domains[k].flags_offset >= 0) wall_words += 3 * size_t(args[k].g.wall_plane);
+        if (domains[k].flags_offset >= 0) wall_words += size_t(args[k].g.nx) * args[k].g.ny * args[k].g.nz;
     if (wall_words > 0) e = cudaMalloc(&b->d_walls, sizeof(uint32_t) * wall_words);
     wall_words = 0;
     for (int k = 0; k < n_domains && e == cudaSuccess; ++k) {
         if (domains[k].flags_offset < 0) continue;
         args[k].g.walls = args[n_domains + k].g.walls = b->d_walls + wall_words;
-        wall_words += 3 * size_t(args[k].g.wall_plane);
+        wall_words += size_t(args[k].g.nx) * args[k].g.ny * args[k].g.nz;
     }
     if (e == cudaSuccess) e = cudaMalloc(&b->d_domains, sizeof(SweepArgs) * args.size());
     if (e == cudaSuccess) e = cudaMalloc(&b->d_tiles, sizeof(BatchTile) * tiles.size());

@@ -56,17 +56,11 @@ LBM_HD constexpr int link_off(int code, int axis) { return ((code >> (8 + 2 * ax
 
 // Wall word of an interior cell, one per cell of a finalized flag field (k_wall_words): bit i (1..26)
 // set when the cell x - c_i that direction i streams from is a NoSlip or UBB cell, so that the sweep
-// replaces population i by the bounced one; the other bits describe the cell and its other links.
-// Two more planes follow the first, read only where WALL_UBB or WALL_PER_LINK asks for them: the
-// directions whose wall is a UBB cell (with WALL_UBB_MIXED and the UBB number in bits 27-28), and the
-// directions whose wall cell is of a per-link type (8 and above).
+// replaces population i by the bounced one; the other bits say what else the cell is next to.
 constexpr uint32_t WALL_SELF = 1u;              // the cell is itself a boundary cell
 constexpr uint32_t WALL_FIXED_DENSITY = 1u << 29;
-constexpr uint32_t WALL_PER_LINK = 1u << 30;
+constexpr uint32_t WALL_PER_LINK = 1u << 30;    // a type with per-link data (8 and above)
 constexpr uint32_t WALL_UBB = 1u << 31;
-constexpr uint32_t WALL_LINKS = 0x07fffffeu;
-constexpr int WALL_UBB_SHIFT = 27;              // second plane: the number of the cell's UBB links ...
-constexpr uint32_t WALL_UBB_MIXED = 1u << 31;   // ... unless they have several
 
 LBM_HD constexpr bool flag_is_ubb(int t) { return t >= FLAG_UBB0 && t < FLAG_UBB0 + MAX_UBB; }
 LBM_HD constexpr bool flag_is_fixed_density(int t) { return t == FLAG_FIXED_DENSITY || t == FLAG_FIXED_DENSITY1; }
@@ -232,10 +226,9 @@ struct Grid {
     // or a fluid cell next to one).  nullptr: every row may.  Sweeps skip the flag loads of the
     // other rows, so that a fluid cell's populations are not held up behind its flag.
     const uint32_t* rowmask;
-    // Wall words of the interior cells, x fastest, in three planes of wall_plane words (see WALL_*);
-    // nullptr: the sweeps take them from the flags.
+    // Wall words of the interior cells, x fastest (see WALL_*); nullptr: the sweeps take the walls
+    // from the flags.
     const uint32_t* walls;
-    unsigned wall_plane;
 };
 
 struct SweepArgs {
@@ -284,65 +277,93 @@ struct NbrOffsets {
     __device__ __forceinline__ int off(int cx, int cy, int cz) const {
         return dx[cx + 1] + dy[cy + 1] + dz[cz + 1];
     }
+    // Offset of the cell x - c of a direction given by its code (direction_code).
+    __device__ __forceinline__ int behind(unsigned code) const {
+        const unsigned cx = code & 3u, cy = (code >> 2) & 3u, cz = code >> 4;
+        return (cx == 0 ? dx[2] : cx == 2 ? dx[0] : 0) + (cy == 0 ? dy[2] : cy == 2 ? dy[0] : 0) +
+               (cz == 0 ? dz[2] : cz == 2 ? dz[0] : 0);
+    }
 };
 
 #ifdef __CUDACC__
-// Directions i of a cell whose source cell x - c_i has a flag type in [lo, hi].  `flags` points at the
-// cell, `fo` holds the flag field's neighbour offsets.  All loads are independent of one another.
-template <int Q>
-__device__ __forceinline__ uint32_t links_into(const uint8_t* flags, const NbrOffsets& fo, int lo, int hi) {
-    using L = Lat<Q>;
-    uint32_t w = 0;
-#pragma unroll
-    for (int i = 1; i < Q; ++i) {
-        const unsigned t = flags[fo.off(-L::cx(i), -L::cy(i), -L::cz(i))] & FLAG_TYPE_MASK;
-        w |= uint32_t(t - unsigned(lo) <= unsigned(hi - lo)) << i;
+// Code of a direction known only at run time: c + 1 per axis, two bits each, x lowest.
+template <int Q> struct DirectionCodes {
+    uint8_t code[Q];
+    constexpr DirectionCodes() : code() {
+        for (int i = 0; i < Q; ++i)
+            code[i] = uint8_t((Lat<Q>::cx(i) + 1) | (Lat<Q>::cy(i) + 1) << 2 | (Lat<Q>::cz(i) + 1) << 4);
     }
-    return w;
+};
+static __constant__ DirectionCodes<19> c_directions19;
+static __constant__ DirectionCodes<27> c_directions27;
+template <int Q> __device__ __forceinline__ unsigned direction_code(int i) {
+    if constexpr (Q == 19) return c_directions19.code[i];
+    else return c_directions27.code[i];
 }
 
-// The same out of line, for sweeps given flags without wall words: one copy per translation unit, and
-// none of its registers in the sweeps.
+// Directions i of a cell whose source cell x - c_i is a NoSlip or UBB cell, from the flags (which point
+// at the cell; the other arguments are the flag field's neighbour offsets).  All loads are independent
+// of one another.  Out of line: one copy per translation unit, and none of its registers in the sweeps.
 template <int Q>
-__device__ __noinline__ uint32_t links_into_far(const uint8_t* flags, int dx0, int dx2, int dy0, int dy2, int dz0,
-                                                int dz2, int lo, int hi) {
+__device__ __noinline__ uint32_t bounce_links(const uint8_t* flags, int dx0, int dx2, int dy0, int dy2, int dz0,
+                                              int dz2) {
+    using L = Lat<Q>;
     NbrOffsets fo;
     fo.dx[0] = dx0; fo.dx[1] = 0; fo.dx[2] = dx2;
     fo.dy[0] = dy0; fo.dy[1] = 0; fo.dy[2] = dy2;
     fo.dz[0] = dz0; fo.dz[1] = 0; fo.dz[2] = dz2;
-    return links_into<Q>(flags, fo, lo, hi);
+    uint32_t w = 0;
+#pragma unroll
+    for (int i = 1; i < Q; ++i) {
+        const int t = flags[fo.off(-L::cx(i), -L::cy(i), -L::cz(i))] & FLAG_TYPE_MASK;
+        w |= uint32_t(t == FLAG_NOSLIP || flag_is_ubb(t)) << i;
+    }
+    return w;
 }
 
-template <int Q>
-__device__ __forceinline__ uint32_t links_from_flags(const Grid& g, int x, int y, int z, int lo, int hi) {
+__device__ __forceinline__ NbrOffsets flag_offsets(const Grid& g, int x, int y, int z) {
     NbrOffsets fo;
     Grid gf = g;
     gf.sy = g.fsy;
     gf.sz = g.fsz;
     fo.init(gf, x, y, z);
-    return links_into_far<Q>(g.flags + ((x + 1) + (y + 1) * g.fsy + (z + 1) * g.fsz), fo.dx[0], fo.dx[2], fo.dy[0],
-                             fo.dy[2], fo.dz[0], fo.dz[2], lo, hi);
+    return fo;
 }
 
-// Wall word of interior cell (x, y, z) for a sweep; 0 away from boundaries.  Links into per-link types
-// bounce back as NoSlip when the plan holds no link tables (then the pre-pass does not run).
-template <int Q>
-__device__ __forceinline__ uint32_t wall_word(const SweepArgs& a, int x, int y, int z) {
-    const Grid& g = a.g;
-    if (g.flags == nullptr || !row_flagged(g, y, z)) return 0;
-    const bool tables = a.link_code != nullptr || a.link_value != nullptr;
-    if (g.walls != nullptr) {
-        const size_t c = unsigned(x) + unsigned(g.nx) * (unsigned(y) + unsigned(g.ny) * unsigned(z));
-        uint32_t w = g.walls[c];
-        if (!tables && (w & WALL_PER_LINK)) w |= g.walls[c + 2 * size_t(g.wall_plane)];
-        return w;
+// Wall word of an interior cell in two parts, with the loads of its populations between them: begin()
+// asks whether the cell's row has walls at all, word() reads the cell's word if so.  A cell in another
+// row, as almost all are, then waits for its populations alone, where the row's answer used to come
+// first.  Without wall words begin() takes them from the flags.
+template <int Q> struct WallProbe {
+    uint32_t from_flags = 0;
+    bool flagged = false;
+    __device__ __forceinline__ void begin(const Grid& g, int x, int y, int z) {
+        if (g.flags == nullptr) return;
+        if (g.walls != nullptr) {
+            flagged = row_flagged(g, y, z);
+            return;
+        }
+        if (!row_flagged(g, y, z)) return;
+        const uint8_t* cell = g.flags + ((x + 1) + (y + 1) * g.fsy + (z + 1) * g.fsz);
+        const int fl = *cell;
+        if (fl & FLAG_TYPE_MASK) from_flags = WALL_SELF;
+        if ((fl & FLAG_TYPE_MASK) || !(fl & FLAG_NEAR_WALL)) return;
+        const NbrOffsets fo = flag_offsets(g, x, y, z);
+        // UBB and per-link links are told apart where they are handled
+        from_flags = bounce_links<Q>(cell, fo.dx[0], fo.dx[2], fo.dy[0], fo.dy[2], fo.dz[0], fo.dz[2]) | WALL_UBB |
+                     WALL_PER_LINK;
     }
-    const int fl = g.flags[(x + 1) + (y + 1) * g.fsy + (z + 1) * g.fsz];
-    if (fl & FLAG_TYPE_MASK) return WALL_SELF;
-    if (!(fl & FLAG_NEAR_WALL)) return 0;
-    uint32_t w = links_from_flags<Q>(g, x, y, z, FLAG_NOSLIP, FLAG_UBB0 + MAX_UBB - 1);
-    if (!tables) w |= links_from_flags<Q>(g, x, y, z, FLAG_FREE_SLIP, FLAG_TYPE_MASK);
-    return w | WALL_UBB;                        // UBB links are told apart where they are handled
+    __device__ __forceinline__ uint32_t word(const Grid& g, int x, int y, int z) const {
+        return flagged ? g.walls[unsigned(x) + unsigned(g.nx) * (unsigned(y) + unsigned(g.ny) * unsigned(z))]
+                       : from_flags;
+    }
+};
+
+template <int Q>
+__device__ __forceinline__ uint32_t wall_word(const Grid& g, int x, int y, int z) {
+    WallProbe<Q> probe;
+    probe.begin(g, x, y, z);
+    return probe.word(g, x, y, z);
 }
 #endif
 

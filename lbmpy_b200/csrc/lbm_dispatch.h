@@ -15,6 +15,13 @@ using MacroLauncher = cudaError_t (*)(const MacroArgs&, dim3, dim3, cudaStream_t
 
 template <class S, class R, int Q, int MK, int PAT>
 cudaError_t launch_sweep(const SweepArgs& a, dim3 grid, dim3 block, cudaStream_t s) {
+    // SRT/TRT pull with FP32 storage runs at memory speed; without the wall code its 48 registers hold the
+    // loads in the better order (D3Q19 512^3: 3.20 ms, with it 3.26 ms).
+    if constexpr (MK == MK_POP && PAT == PAT_PULL && std::is_same<S, float>::value)
+        if (a.g.flags == nullptr) {
+            k_sweep<S, R, Q, MK, PAT, false><<<grid, block, 0, s>>>(a);
+            return cudaGetLastError();
+        }
     k_sweep<S, R, Q, MK, PAT><<<grid, block, 0, s>>>(a);
     return cudaGetLastError();
 }

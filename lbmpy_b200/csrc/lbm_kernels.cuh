@@ -101,17 +101,35 @@ template <class S> __device__ __forceinline__ S* at(S* field, unsigned slot_off,
                                 size_t(unsigned(cell_off) * unsigned(sizeof(S))));
 }
 
-// The slots of a field in order.  With the field's strides in kernel parameters a slot's address is
-// uniform arithmetic; read from shared memory they are ordinary registers, where the compiler keeps the
-// products of all slots from the loads to the stores and spills: there the address is walked, hidden
-// from it step by step.
-template <class S, bool WALK> struct Slots {
+// How a sweep addresses the slots of a field.
+//   ADDR_INDEX    one 32-bit element index per access: the least work ahead of the first load, for the
+//                 SRT/TRT sweeps, which run at memory speed (D3Q19 TRT pull FP32 256^3: 402 us, with
+//                 uniform addresses 406 us)
+//   ADDR_UNIFORM  slot part uniform, cell part shared by the slots of one offset (at()): fewer
+//                 instructions, for the methods limited by their number (D3Q27 cumulant AA FP32
+//                 256x128x128: 164.6 -> 157.8 us, D3Q19 MRT pull FP32 256^3: 521 -> 493 us, both with
+//                 the FP32 copies of the physics)
+//   ADDR_WALK     strides read from shared memory (batched sweep) are ordinary registers, where the
+//                 compiler keeps the products of all slots from the loads to the stores and spills:
+//                 the slot address is walked, hidden from it step by step (D3Q19 MRT batch at 80
+//                 registers: 48 -> 40 bytes of stack, SRT/TRT none)
+__device__ __forceinline__ unsigned eidx(unsigned slot_off, int cell_off) { return slot_off + unsigned(cell_off); }
+
+enum : int { ADDR_INDEX = 0, ADDR_UNIFORM = 1, ADDR_WALK = 2 };
+template <int MK> struct AddrOf { static constexpr int value = MK == MK_POP ? ADDR_INDEX : ADDR_UNIFORM; };
+
+template <int ADDR, class S> __device__ __forceinline__ S* addr(S* field, unsigned slot_off, int cell_off) {
+    if constexpr (ADDR == ADDR_INDEX) return field + eidx(slot_off, cell_off);
+    else return at(field, slot_off, cell_off);
+}
+
+template <class S, int ADDR> struct Slots {
     S* field;
     unsigned sq;
     __device__ __forceinline__ Slots(S* f, unsigned stride) : field(f), sq(stride) {}
     // Address of (slot, cell offset); slots must be taken in ascending order, without gaps from 0.
     __device__ __forceinline__ S* operator()(int slot, int cell_off) {
-        if constexpr (WALK) {
+        if constexpr (ADDR == ADDR_WALK) {
             if (slot > 0) {
                 field += sq;
                 asm volatile("" : "+l"(field));
@@ -166,27 +184,59 @@ __device__ __forceinline__ R load_f_out(const SweepArgs& a, int x, int y, int z,
 // ends every warp of a cavity has one.  The directions come as one word per cell (`w`, wall_word), so
 // the bounced populations are fetched together after a single load, where a flag per neighbour cost
 // up to Q - 1 dependent round trips, one after another.
-template <class S, class R, int Q, int PAT, bool SHARED_ARGS = false>
+template <class S, class R, int Q, int PAT, int ADDR>
 __device__ __forceinline__ void bounce_back(R (&f)[Q], const SweepArgs& a, const NbrOffsets& nb, int cell,
                                          int x, int y, int z, uint32_t w) {
     using L = Lat<Q>;
     using PA = Access<PrevPattern<PAT>::value>;
     const Grid& g = a.g;
     const S* src = static_cast<const S*>(a.src);
+    uint32_t um = 0;            // directions from UBB cells
+    unsigned numbers = 0;       // bit t: a UBB cell of type t among them
+    if (w & (WALL_UBB | WALL_PER_LINK)) {
+        // Which links these are, one at a time: few cells have any, and loading the types of all links
+        // at once would cost every cell of the sweep the registers.  Per-link types bounce back as
+        // NoSlip when the plan holds no link tables (then the pre-pass does not run).
+        const bool tables = a.link_code != nullptr || a.link_value != nullptr;
+        const NbrOffsets fo = flag_offsets(g, x, y, z);
+        const uint8_t* fl = g.flags + ((x + 1) + (y + 1) * g.fsy + (z + 1) * g.fsz);
+        uint32_t todo = (w & WALL_PER_LINK) && !tables ? ((1u << Q) - 2u) : (w & ((1u << Q) - 2u));
+#pragma unroll 1
+        while (todo != 0) {
+            const int i = __ffs(int(todo)) - 1;
+            todo &= todo - 1u;
+            const int t = fl[fo.behind(direction_code<Q>(i))] & FLAG_TYPE_MASK;
+            if (flag_is_ubb(t)) {
+                um |= 1u << i;
+                numbers |= 1u << t;
+            }
+            if (t >= FLAG_FREE_SLIP && !tables) w |= 1u << i;
+        }
+    }
+    if constexpr (ADDR == ADDR_INDEX) {
+#pragma unroll
+        for (int i = 1; i < Q; ++i) {
+            if (!((w >> i) & 1u)) continue;
+            // f_out(x, inv i): where the previous step wrote direction inv(i) of this cell
+            const int j = L::inv(i);
+            const int off = nb.off(PA::template woff<Q>(j, 0), PA::template woff<Q>(j, 1), PA::template woff<Q>(j, 2));
+            f[i] = Conv<S, R>::ld(src + eidx(PA::template wslot<Q>(j) * g.sq, cell + off));
+        }
+    } else {
+        Slots<const S, ADDR> slots(src, g.sq);
+#pragma unroll
+        for (int s = 0; s < Q; ++s) {
+            // slot s holds f_out(x, j), which replaces direction i = inv(j): where the previous step
+            // wrote direction j of this cell (its slot rule is its own inverse)
+            const int j = PA::template wslot<Q>(s), i = L::inv(j);
+            const int off = nb.off(PA::template woff<Q>(j, 0), PA::template woff<Q>(j, 1), PA::template woff<Q>(j, 2));
+            const S* q = slots(s, cell + off);
+            if (i > 0 && ((w >> i) & 1u)) f[i] = Conv<S, R>::ld(q);
+        }
+    }
+    if (um == 0) return;
     // Interior cell indices fit 32 bits (the host bounds the field below 2^32 elements).
     const unsigned icell = unsigned(x) + unsigned(g.nx) * (unsigned(y) + unsigned(g.ny) * unsigned(z));
-    Slots<const S, SHARED_ARGS> slots(src, g.sq);
-#pragma unroll
-    for (int s = 0; s < Q; ++s) {
-        // slot s holds f_out(x, j), which replaces direction i = inv(j): where the previous step
-        // wrote direction j of this cell (its slot rule is its own inverse)
-        const int j = PA::template wslot<Q>(s), i = L::inv(j);
-        const int off = nb.off(PA::template woff<Q>(j, 0), PA::template woff<Q>(j, 1), PA::template woff<Q>(j, 2));
-        const S* q = slots(s, cell + off);
-        if (i > 0 && ((w >> i) & 1u)) f[i] = Conv<S, R>::ld(q);
-    }
-    if (!(w & WALL_UBB)) return;
-    const uint32_t um = g.walls != nullptr ? g.walls[size_t(g.wall_plane) + icell] : (w | WALL_UBB_MIXED);
     // compressible: the prescribed wall density, else the cell's density at the previous step,
     // gathered before the sweep (k_ubb_density; in-place sweeps overwrite the values it is summed
     // from)
@@ -197,26 +247,21 @@ __device__ __forceinline__ void bounce_back(R (&f)[Q], const SweepArgs& a, const
         ux = R(uw[0]); uy = R(uw[1]); uz = R(uw[2]);
         if ((a.p.ubb_adapt_mask >> u) & 1u) {   // the equilibrium velocity of the wall
             const R h = R(0.5) / rho;
-            ux -= h * R(a.p.force[0]); uy -= h * R(a.p.force[1]); uz -= h * R(a.p.force[2]);
+            ux -= h * p_force<R>(a.p, 0); uy -= h * p_force<R>(a.p, 1); uz -= h * p_force<R>(a.p, 2);
         }
     };
-    const bool each = (um & WALL_UBB_MIXED) != 0 || a.p.ubb_link_mask != 0;
+    const bool each = (numbers & (numbers - 1u)) != 0 || a.p.ubb_link_mask != 0;
     if (!each) {                                // one wall with one velocity
-        const int u = (um >> WALL_UBB_SHIFT) & 3u;
+        const int u = __ffs(int(numbers)) - 1 - FLAG_UBB0;
         wall(u, a.p.ubb[u]);
     }
 #pragma unroll
     for (int i = 1; i < Q; ++i) {
         if (!((um >> i) & 1u)) continue;
         if (each) {
-            Grid gf = g;
-            gf.sy = g.fsy;
-            gf.sz = g.fsz;
-            NbrOffsets fo;
-            fo.init(gf, x, y, z);
+            const NbrOffsets fo = flag_offsets(g, x, y, z);
             const int u = (g.flags[(x + 1) + (y + 1) * g.fsy + (z + 1) * g.fsz +
                                    fo.off(-L::cx(i), -L::cy(i), -L::cz(i))] & FLAG_TYPE_MASK) - FLAG_UBB0;
-            if (unsigned(u) >= unsigned(MAX_UBB)) continue;
             // per-link velocity of the link x -> x - c_i (direction inv i)
             wall(u, ((a.p.ubb_link_mask >> u) & 1u)
                         ? a.ubb_link_vel + (size_t(a.ubb_block[icell]) * Q + size_t(L::inv(i))) * 3 : a.p.ubb[u]);
@@ -228,17 +273,22 @@ __device__ __forceinline__ void bounce_back(R (&f)[Q], const SweepArgs& a, const
 
 // The whole update of one cell: pull through the accessor, fused bounce-back, collision, push
 // through the accessor.  Shared by the single-domain and the batched sweeps.
-template <class S, class R, int Q, int MK, int PAT, bool SHARED_ARGS = false>
+template <class S, class R, int Q, int MK, int PAT, int ADDR = AddrOf<MK>::value, bool WALLS = true>
 __device__ __forceinline__ void sweep_cell(const SweepArgs& a, int x, int y, int z) {
     using A = Access<PAT>;
     const Grid& g = a.g;
-    // Wall word first or together with the populations.  Every address below lies inside the
-    // ghost-inclusive field whatever the cell type, so the populations can be loaded before the
-    // word is known: a boundary cell wastes a few loads, and no cell waits for a round trip
-    // before its loads issue.  The specialised cumulant sweep keeps the word first: its register
-    // budget (64 per thread for AA) does not hold it alongside 27 loads in flight.
-    constexpr bool word_first = MK == MK_CUM1 || MK == MK_CUM1_MLP;
-    const uint32_t w = wall_word<Q>(a, x, y, z);
+    // Every address below lies inside the ghost-inclusive field whatever the cell type, so the
+    // populations are loaded before the wall word is known: a boundary cell wastes a few loads, and
+    // no cell waits for a round trip before its loads issue.  Two exceptions.  The specialised cumulant
+    // sweep asks for the word and looks at it first: its register budget (64 per thread) does not hold
+    // it alongside 27 loads in flight.  The SRT/TRT sweeps ask for it ahead of the populations: with the
+    // row's answer looked at behind them, the periodic box, which runs at memory speed, loses 2 %
+    // (D3Q19 TRT pull FP32 512^3).
+    constexpr bool word_first = MK == MK_CUM1 || MK == MK_CUM1_MLP, word_early = MK == MK_POP;
+    WallProbe<Q> probe;
+    if (WALLS) probe.begin(g, x, y, z);
+    uint32_t w = 0;
+    if (WALLS && (word_first || word_early)) w = probe.word(g, x, y, z);
     if (word_first && (w & WALL_SELF)) return;
     NbrOffsets nb;
     nb.init(g, x, y, z);
@@ -246,22 +296,39 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs& a, int x, int y, int
     const S* src = static_cast<const S*>(a.src);
     S* dst = static_cast<S*>(a.dst);
     R f[Q];
-    Slots<const S, SHARED_ARGS> rs(src, g.sq);
+    if constexpr (ADDR == ADDR_INDEX) {
 #pragma unroll
-    for (int s = 0; s < Q; ++s) {
-        const int i = A::template rslot<Q>(s);       // the slot rule is its own inverse
-        const int off = nb.off(A::template roff<Q>(i, 0), A::template roff<Q>(i, 1), A::template roff<Q>(i, 2));
-        f[i] = Conv<S, R>::ld(rs(s, cell + off));
+        for (int i = 0; i < Q; ++i) {
+            const int off = nb.off(A::template roff<Q>(i, 0), A::template roff<Q>(i, 1), A::template roff<Q>(i, 2));
+            f[i] = Conv<S, R>::ld(src + eidx(A::template rslot<Q>(i) * g.sq, cell + off));
+        }
+    } else {
+        Slots<const S, ADDR> rs(src, g.sq);
+#pragma unroll
+        for (int s = 0; s < Q; ++s) {
+            const int i = A::template rslot<Q>(s);       // the slot rule is its own inverse
+            const int off = nb.off(A::template roff<Q>(i, 0), A::template roff<Q>(i, 1), A::template roff<Q>(i, 2));
+            f[i] = Conv<S, R>::ld(rs(s, cell + off));
+        }
     }
-    if (!word_first && (w & WALL_SELF)) return;
-    if (w != 0) bounce_back<S, R, Q, PAT, SHARED_ARGS>(f, a, nb, cell, x, y, z, w);
+    if (WALLS && !word_first && !word_early) w = probe.word(g, x, y, z);
+    if (WALLS && (w & WALL_SELF)) return;
+    if (WALLS && w != 0) bounce_back<S, R, Q, PAT, ADDR>(f, a, nb, cell, x, y, z, w);
     const R om = collide<R, Q, MK>(f, a.p);
-    Slots<S, SHARED_ARGS> ws(dst, g.sq);
+    if constexpr (ADDR == ADDR_INDEX) {
 #pragma unroll
-    for (int s = 0; s < Q; ++s) {
-        const int i = A::template wslot<Q>(s);
-        const int off = nb.off(A::template woff<Q>(i, 0), A::template woff<Q>(i, 1), A::template woff<Q>(i, 2));
-        Conv<S, R>::st(ws(s, cell + off), f[i]);
+        for (int i = 0; i < Q; ++i) {
+            const int off = nb.off(A::template woff<Q>(i, 0), A::template woff<Q>(i, 1), A::template woff<Q>(i, 2));
+            Conv<S, R>::st(dst + eidx(A::template wslot<Q>(i) * g.sq, cell + off), f[i]);
+        }
+    } else {
+        Slots<S, ADDR> ws(dst, g.sq);
+#pragma unroll
+        for (int s = 0; s < Q; ++s) {
+            const int i = A::template wslot<Q>(s);
+            const int off = nb.off(A::template woff<Q>(i, 0), A::template woff<Q>(i, 1), A::template woff<Q>(i, 2));
+            Conv<S, R>::st(ws(s, cell + off), f[i]);
+        }
     }
     if (a.omega_out != nullptr) a.omega_out[x + g.nx * (y + (long long)g.ny * z)] = (float)om;
 }
@@ -274,6 +341,8 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs& a, int x, int y, int
 // for spills with -Xptxas -v: 80 (3 blocks), 64 (4) and 48 (5).
 template <class S, int Q, int MK, int PAT> struct SweepMinBlocks { static constexpr int value = 1; };
 template <> struct SweepMinBlocks<float, 27, MK_CUM1, PAT_AA_ODD> { static constexpr int value = 4; };
+template <> struct SweepMinBlocks<double, 19, MK_POP, PAT_PULL> { static constexpr int value = 2; };
+template <> struct SweepMinBlocks<float, 27, MK_CUM1, PAT_PULL> { static constexpr int value = 4; };
 template <> struct SweepMinBlocks<float, 27, MK_CUM1, PAT_AA_EVEN> { static constexpr int value = 4; };
 template <> struct SweepMinBlocks<float, 19, MK_POP, PAT_PULL> { static constexpr int value = 5; };
 template <> struct SweepMinBlocks<float, 19, MK_POP, PAT_AA_ODD> { static constexpr int value = 4; };
@@ -283,13 +352,14 @@ template <> struct SweepMinBlocks<float, 27, MK_POP, PAT_AA_EVEN> { static const
 template <> struct SweepMinBlocks<float, 19, MK_MRT, PAT_PULL> { static constexpr int value = 4; };
 template <> struct SweepMinBlocks<float, 27, MK_MRT, PAT_PULL> { static constexpr int value = 3; };
 
-template <class S, class R, int Q, int MK, int PAT>
+// WALLS false: for domains without flags.
+template <class S, class R, int Q, int MK, int PAT, bool WALLS = true>
 __global__ void __launch_bounds__(256, SweepMinBlocks<S, Q, MK, PAT>::value) k_sweep(const SweepArgs a) {
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     const int y = blockIdx.y * blockDim.y + threadIdx.y;
     const int z = blockIdx.z;
     if (x >= a.g.nx || y >= a.g.ny) return;
-    sweep_cell<S, R, Q, MK, PAT>(a, x, y, z);
+    sweep_cell<S, R, Q, MK, PAT, AddrOf<MK>::value, WALLS>(a, x, y, z);
 }
 
 // Pipelined z-columns: each thread sweeps a.zc consecutive cells along z and issues the loads of
@@ -310,7 +380,7 @@ __global__ void __launch_bounds__(256, 2) k_sweep_zpipe(const SweepArgs a) {
     const S* src = static_cast<const S*>(a.src);
     S* dst = static_cast<S*>(a.dst);
     auto load = [&](int z, R (&h)[Q], uint32_t& hw) {
-        hw = wall_word<Q>(a, x, y, z);
+        hw = wall_word<Q>(g, x, y, z);
         NbrOffsets nb;
         nb.init(g, x, y, z);
         const int cell = (x + 1) + (y + 1) * g.sy + (z + 1) * g.sz;
@@ -334,7 +404,7 @@ __global__ void __launch_bounds__(256, 2) k_sweep_zpipe(const SweepArgs a) {
         NbrOffsets nb;
         nb.init(g, x, y, z);
         const int cell = (x + 1) + (y + 1) * g.sy + (z + 1) * g.sz;
-        if (w != 0) bounce_back<S, R, Q, PAT>(f, a, nb, cell, x, y, z, w);
+        if (w != 0) bounce_back<S, R, Q, PAT, AddrOf<MK>::value>(f, a, nb, cell, x, y, z, w);
         collide<R, Q, MK>(f, a.p);
 #pragma unroll
         for (int i = 0; i < Q; ++i) {
@@ -369,15 +439,23 @@ __device__ __forceinline__ void prefetch_cell(const SweepArgs& a, int x, int y, 
 // registers, so they are summed here first, for every pattern.
 template <class S, class R, int Q, int PAT>
 __global__ void __launch_bounds__(256) k_ubb_density(const SweepArgs a, R* rho_out) {
+    using L = Lat<Q>;
     using PA = Access<PrevPattern<PAT>::value>;
     const Grid& g = a.g;
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     const int y = blockIdx.y * blockDim.y + threadIdx.y;
     const int z = blockIdx.z;
     if (x >= g.nx || y >= g.ny) return;
-    const uint32_t w = wall_word<Q>(a, x, y, z);
-    if (!(w & WALL_UBB)) return;
-    if (g.walls == nullptr && links_from_flags<Q>(g, x, y, z, FLAG_UBB0, FLAG_UBB0 + MAX_UBB - 1) == 0) return;
+    if (!(wall_word<Q>(g, x, y, z) & WALL_UBB)) return;
+    if (g.walls == nullptr) {
+        const NbrOffsets fo = flag_offsets(g, x, y, z);
+        const uint8_t* fl = g.flags + ((x + 1) + (y + 1) * g.fsy + (z + 1) * g.fsz);
+        bool moving = false;
+#pragma unroll
+        for (int i = 1; i < Q; ++i)
+            if (flag_is_ubb(fl[fo.off(-L::cx(i), -L::cy(i), -L::cz(i))] & FLAG_TYPE_MASK)) moving = true;
+        if (!moving) return;
+    }
     NbrOffsets nb;
     nb.init(g, x, y, z);
     const int cell = (x + 1) + (y + 1) * g.sy + (z + 1) * g.sz;
@@ -437,7 +515,7 @@ __global__ void __launch_bounds__(256, BatchMinBlocks<S, Q, MK>::value) k_sweep_
         if (x < sa.g.nx && y < sa.g.ny) {
             const int z1 = min(tile.z0 + b.cells_z, sa.g.nz);
 #pragma unroll 1
-            for (int z = tile.z0; z < z1; ++z) sweep_cell<S, R, Q, MK, PAT, true>(sa, x, y, z);
+            for (int z = tile.z0; z < z1; ++z) sweep_cell<S, R, Q, MK, PAT, ADDR_WALK>(sa, x, y, z);
         }
     }
 }
@@ -615,7 +693,7 @@ __global__ void __launch_bounds__(256) k_boundary_prepass(const SweepArgs a) {
     if (x >= g.nx || y >= g.ny || !row_flagged(g, y, z)) return;
     const int fcell = (x + 1) + (y + 1) * g.fsy + (z + 1) * g.fsz;
     if (g.walls != nullptr) {
-        if (!(wall_word<Q>(a, x, y, z) & (WALL_FIXED_DENSITY | WALL_PER_LINK))) return;
+        if (!(wall_word<Q>(g, x, y, z) & (WALL_FIXED_DENSITY | WALL_PER_LINK))) return;
     } else {
         const int fl = g.flags[fcell];
         if ((fl & FLAG_TYPE_MASK) || !(fl & FLAG_NEAR_WALL)) return;

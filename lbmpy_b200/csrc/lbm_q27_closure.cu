@@ -65,7 +65,8 @@ __global__ void __launch_bounds__(256, 3) k_sweep_closure_tc(const SweepArgs a) 
 #pragma unroll 1
     for (int z = z0; z < z1; ++z) {
         if (z + 1 < z1) prefetch_cell<float, 27, PAT>(a, x, y, z + 1);
-        const uint32_t w = wall_word<27>(a, x, y, z);
+        WallProbe<27> probe;
+        probe.begin(g, x, y, z);
         NbrOffsets nb;
         nb.init(g, x, y, z);
         const int cell = (x + 1) + (y + 1) * g.sy + (z + 1) * g.sz;
@@ -75,8 +76,9 @@ __global__ void __launch_bounds__(256, 3) k_sweep_closure_tc(const SweepArgs a) 
             const int off = nb.off(A::template roff<27>(i, 0), A::template roff<27>(i, 1), A::template roff<27>(i, 2));
             f[i] = *at(src, A::template rslot<27>(i) * g.sq, cell + off);
         }
+        const uint32_t w = probe.word(g, x, y, z);
         const bool fluid = inside && !(w & WALL_SELF);
-        if (fluid && w != 0) bounce_back<float, float, 27, PAT>(f, a, nb, cell, x, y, z, w);
+        if (fluid && w != 0) bounce_back<float, float, 27, PAT, ADDR_UNIFORM>(f, a, nb, cell, x, y, z, w);
         __syncwarp();
         const float om = collide_cum_ho1<float, true>(f, a.p, nu);
         if (fluid) {

@@ -58,6 +58,7 @@ __global__ void __launch_bounds__(32 * QUAD_ROWS, 4) k_sweep_quad(const SweepArg
     static_assert(PAT == PAT_PULL || PAT == PAT_AA_EVEN || PAT == PAT_AA_ODD, "quad sweep: pull and AA");
     using L = Lat<Q>;
     using A = Access<PAT>;
+    constexpr int ADDR = AddrOf<MK>::value;
     const Grid& g = a.g;
     const int lane = threadIdx.x;
     const int quads_per_row = g.nx >> 2;
@@ -77,11 +78,9 @@ __global__ void __launch_bounds__(32 * QUAD_ROWS, 4) k_sweep_quad(const SweepArg
     const S* src = static_cast<const S*>(a.src);
     S* dst = static_cast<S*>(a.dst);
 
-    uint32_t w[4] = {0, 0, 0, 0};
-    if (g.flags != nullptr && row_flagged(g, y, z)) {
+    WallProbe<Q> probe[4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) w[k] = wall_word<Q>(a, x0 + k, y, z);
-    }
+    for (int k = 0; k < 4; ++k) probe[k].begin(g, x0 + k, y, z);
 
     F2 f0[Q], f1[Q];     // cells (x0, x0+1) and (x0+2, x0+3)
 #pragma unroll
@@ -90,23 +89,26 @@ __global__ void __launch_bounds__(32 * QUAD_ROWS, 4) k_sweep_quad(const SweepArg
         const int yz = nbA.off(0, A::template roff<Q>(i, 1), A::template roff<Q>(i, 2));
         const unsigned slot = A::template rslot<Q>(i) * g.sq;
         float P[4];
-        quad_ld<S>(at(src, slot, cellA + yz), P);
+        quad_ld<S>(addr<ADDR>(src, slot, cellA + yz), P);
         float v[4];
         if (cx == 0) {
             v[0] = P[0]; v[1] = P[1]; v[2] = P[2]; v[3] = P[3];
         } else if (cx == -1) {                     // cells read x - 1: (x0 - 1 .. x0 + 2)
             float up = __shfl_up_sync(0xffffffffu, P[3], 1);
-            if (lane == 0) up = Conv<S, float>::ld(at(src, slot, cellA + yz + nbA.dx[0]));
+            if (lane == 0) up = Conv<S, float>::ld(addr<ADDR>(src, slot, cellA + yz + nbA.dx[0]));
             v[0] = up; v[1] = P[0]; v[2] = P[1]; v[3] = P[2];
         } else {                                   // cells read x + 1: (x0 + 1 .. x0 + 4)
             float dn = __shfl_down_sync(0xffffffffu, P[0], 1);
-            if (lane == last_lane) dn = Conv<S, float>::ld(at(src, slot, cellA + 3 + yz + nbD.dx[2]));
+            if (lane == last_lane) dn = Conv<S, float>::ld(addr<ADDR>(src, slot, cellA + 3 + yz + nbD.dx[2]));
             v[0] = P[1]; v[1] = P[2]; v[2] = P[3]; v[3] = dn;
         }
         f0[i] = F2(v[0], v[1]);
         f1[i] = F2(v[2], v[3]);
     }
     // cells next to a boundary: per-cell fused bounce-back on the scalar path
+    uint32_t w[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) w[k] = probe[k].word(g, x0 + k, y, z);
     if ((w[0] | w[1] | w[2] | w[3]) & ~WALL_SELF) {
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
@@ -119,7 +121,7 @@ __global__ void __launch_bounds__(32 * QUAD_ROWS, 4) k_sweep_quad(const SweepArg
             }
             NbrOffsets nb;
             nb.init(g, x0 + k, y, z);
-            bounce_back<S, float, Q, PAT>(t, a, nb, cellA + k, x0 + k, y, z, w[k]);
+            bounce_back<S, float, Q, PAT, ADDR>(t, a, nb, cellA + k, x0 + k, y, z, w[k]);
 #pragma unroll
             for (int i = 0; i < Q; ++i) {
                 F2& h = k < 2 ? f0[i] : f1[i];
@@ -129,16 +131,20 @@ __global__ void __launch_bounds__(32 * QUAD_ROWS, 4) k_sweep_quad(const SweepArg
     }
     collide2<float, Q, MK>(f0, a.p);
     collide2<float, Q, MK>(f1, a.p);
-    // Non-fluid cells leave their own slots as they are in AA even steps (neighbours read them in
-    // the fused bounce-back): slot inv(i) is rewritten with its current value.
-    if (PAT == PAT_AA_EVEN && ((w[0] | w[1] | w[2] | w[3]) & WALL_SELF)) {
+    // A boundary cell leaves the field as it is (see the pair sweep).
+    if (PAT != PAT_PULL && ((w[0] | w[1] | w[2] | w[3]) & WALL_SELF)) {
 #pragma unroll
-        for (int i = 0; i < Q; ++i) {
-            const S* q = at(src, L::inv(i) * g.sq, cellA);
-            if (w[0] & WALL_SELF) f0[i].v.x = Conv<S, float>::ld(q);
-            if (w[1] & WALL_SELF) f0[i].v.y = Conv<S, float>::ld(q + 1);
-            if (w[2] & WALL_SELF) f1[i].v.x = Conv<S, float>::ld(q + 2);
-            if (w[3] & WALL_SELF) f1[i].v.y = Conv<S, float>::ld(q + 3);
+        for (int k = 0; k < 4; ++k) {
+            if (!(w[k] & WALL_SELF)) continue;
+            NbrOffsets nb;
+            nb.init(g, x0 + k, y, z);
+#pragma unroll
+            for (int i = 0; i < Q; ++i) {
+                const int off = nb.off(A::template woff<Q>(i, 0), A::template woff<Q>(i, 1), A::template woff<Q>(i, 2));
+                const float v = Conv<S, float>::ld(addr<ADDR>(src, A::template wslot<Q>(i) * g.sq, cellA + k + off));
+                F2& h = k < 2 ? f0[i] : f1[i];
+                if (k & 1) h.v.y = v; else h.v.x = v;
+            }
         }
     }
 
@@ -149,32 +155,32 @@ __global__ void __launch_bounds__(32 * QUAD_ROWS, 4) k_sweep_quad(const SweepArg
         const unsigned slot = A::template wslot<Q>(i) * g.sq;
         const float va = f0[i].v.x, vb = f0[i].v.y, vc = f1[i].v.x, vd = f1[i].v.y;
         if (cx == 0) {
-            if (active) quad_st<S>(at(dst, slot, cellA + yz), va, vb, vc, vd);
+            if (active) quad_st<S>(addr<ADDR>(dst, slot, cellA + yz), va, vb, vc, vd);
         } else if (cx == 1) {                      // A..D -> x0+1 .. x0+4
             const float prevD = __shfl_up_sync(0xffffffffu, vd, 1);
             if (active) {
                 if (lane == 0) {                   // x0 belongs to the previous warp's last lane
-                    S* p = at(dst, slot, cellA + yz);
+                    S* p = addr<ADDR>(dst, slot, cellA + yz);
                     Conv<S, float>::st(p + 1, va);
                     Conv<S, float>::st(p + 2, vb);
                     Conv<S, float>::st(p + 3, vc);
                 } else {
-                    quad_st<S>(at(dst, slot, cellA + yz), prevD, va, vb, vc);
+                    quad_st<S>(addr<ADDR>(dst, slot, cellA + yz), prevD, va, vb, vc);
                 }
-                if (lane == last_lane) Conv<S, float>::st(at(dst, slot, cellA + 3 + yz + nbD.dx[2]), vd);
+                if (lane == last_lane) Conv<S, float>::st(addr<ADDR>(dst, slot, cellA + 3 + yz + nbD.dx[2]), vd);
             }
         } else {                                   // A..D -> x0-1 .. x0+2
             const float nextA = __shfl_down_sync(0xffffffffu, va, 1);
             if (active) {
                 if (lane == last_lane) {           // x0+3 belongs to the next warp's lane 0
-                    S* p = at(dst, slot, cellA + yz);
+                    S* p = addr<ADDR>(dst, slot, cellA + yz);
                     Conv<S, float>::st(p, vb);
                     Conv<S, float>::st(p + 1, vc);
                     Conv<S, float>::st(p + 2, vd);
                 } else {
-                    quad_st<S>(at(dst, slot, cellA + yz), vb, vc, vd, nextA);
+                    quad_st<S>(addr<ADDR>(dst, slot, cellA + yz), vb, vc, vd, nextA);
                 }
-                if (lane == 0) Conv<S, float>::st(at(dst, slot, cellA + yz + nbA.dx[0]), va);
+                if (lane == 0) Conv<S, float>::st(addr<ADDR>(dst, slot, cellA + yz + nbA.dx[0]), va);
             }
         }
     }

@@ -222,7 +222,7 @@ __global__ void __launch_bounds__(W) k_sweep_staged(const SweepArgs a, const int
         staged::arrive(bar);
     };
     auto word_of = [&](const StagedTile& t) -> uint32_t {
-        return tid < t.w ? wall_word<Q>(a, t.xs + tid, t.y, t.z) : 0u;
+        return tid < t.w ? wall_word<Q>(g, t.xs + tid, t.y, t.z) : 0u;
     };
 
     const int npro = min(ns, mine);
@@ -268,7 +268,7 @@ __global__ void __launch_bounds__(W) k_sweep_staged(const SweepArgs a, const int
             NbrOffsets nb;
             nb.init(g, x, t.y, t.z);
             const int cell = (x + 1) + (t.y + 1) * g.sy + (t.z + 1) * g.sz;
-            if (w != 0) bounce_back<S, R, Q, PAT>(f, a, nb, cell, x, t.y, t.z, w);
+            if (w != 0) bounce_back<S, R, Q, PAT, AddrOf<MK>::value>(f, a, nb, cell, x, t.y, t.z, w);
             const R om = collide<R, Q, MK>(f, a.p);
 #pragma unroll
             for (int i = 0; i < Q; ++i) {
