@@ -375,8 +375,7 @@ using UbbLauncher = cudaError_t (*)(const SweepArgs&, void*, dim3, dim3, cudaStr
 
 template <class S, class R, int Q, int PAT>
 cudaError_t launch_ubb(const SweepArgs& a, void* out, dim3 grid, dim3 block, cudaStream_t s) {
-    k_ubb_density<S, R, Q, PAT><<<grid, block, 0, s>>>(a, static_cast<R*>(out));
-    return cudaGetLastError();
+    return launch_chained(&k_ubb_density<S, R, Q, PAT>, grid, block, 0, s, a, static_cast<R*>(out));
 }
 
 template <class S, class R, int Q>
@@ -1132,8 +1131,8 @@ cudaError_t launch_sparse_get(const SparseArgs& a, double* rho, double* u, cudaS
 template <class S, class R, int Q>
 cudaError_t launch_sparse_ubb(const SparseArgs& a, const uint32_t* links, int64_t n, const double* u,
                               cudaStream_t s) {
-    k_sparse_ubb<S, R, Q><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(a, links, (long long)n, u[0], u[1], u[2]);
-    return cudaGetLastError();
+    return launch_chained(&k_sparse_ubb<S, R, Q>, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, s, a, links,
+                          (long long)n, u[0], u[1], u[2]);
 }
 
 int sparse_common(const LbmPlan* p, const void* src, const void* dst, int64_t n_fluid, int64_t n_cells,

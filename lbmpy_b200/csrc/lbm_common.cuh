@@ -365,6 +365,15 @@ __device__ __forceinline__ uint32_t wall_word(const Grid& g, int x, int y, int z
     probe.begin(g, x, y, z);
     return probe.word(g, x, y, z);
 }
+
+// Sweeps are chained: each is launched while the one before it in its stream still runs (dispatch.h) and
+// waits here, before its first access to memory, until that one has completed and its writes are
+// visible.  The launch itself and the ramp of the blocks are then hidden; for domains of a few thousand
+// cells they are a third of a step.
+__device__ __forceinline__ void chain_wait() {
+    asm volatile("griddepcontrol.launch_dependents;");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
 #endif
 
 }  // namespace lbm

@@ -13,17 +13,30 @@ namespace lbm {
 using SweepLauncher = cudaError_t (*)(const SweepArgs&, dim3, dim3, cudaStream_t);
 using MacroLauncher = cudaError_t (*)(const MacroArgs&, dim3, dim3, cudaStream_t);
 
+// Launches a kernel that begins with chain_wait(): it may start while the kernel before it in the stream
+// still runs, and waits for it there.
+template <class... KA, class... A>
+cudaError_t launch_chained(void (*kernel)(KA...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, const A&... args) {
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c = {};
+    c.gridDim = grid;
+    c.blockDim = block;
+    c.dynamicSmemBytes = smem;
+    c.stream = s;
+    c.attrs = &attr;
+    c.numAttrs = 1;
+    return cudaLaunchKernelEx(&c, kernel, KA(args)...);
+}
+
 template <class S, class R, int Q, int MK, int PAT>
 cudaError_t launch_sweep(const SweepArgs& a, dim3 grid, dim3 block, cudaStream_t s) {
     // SRT/TRT pull with FP32 storage runs at memory speed; without the wall code its 48 registers hold the
     // loads in the better order (D3Q19 512^3: 3.20 ms, with it 3.26 ms).
     if constexpr (MK == MK_POP && PAT == PAT_PULL && std::is_same<S, float>::value)
-        if (a.g.flags == nullptr) {
-            k_sweep<S, R, Q, MK, PAT, false><<<grid, block, 0, s>>>(a);
-            return cudaGetLastError();
-        }
-    k_sweep<S, R, Q, MK, PAT><<<grid, block, 0, s>>>(a);
-    return cudaGetLastError();
+        if (a.g.flags == nullptr) return launch_chained(&k_sweep<S, R, Q, MK, PAT, false>, grid, block, 0, s, a);
+    return launch_chained(&k_sweep<S, R, Q, MK, PAT>, grid, block, 0, s, a);
 }
 
 template <class S, class R, int Q, int MK, int PAT>
@@ -34,8 +47,7 @@ cudaError_t launch_set_eq(const MacroArgs& a, dim3 grid, dim3 block, cudaStream_
 
 template <class S, int Q, int MK, int PAT>
 cudaError_t launch_sweep_pair(const SweepArgs& a, dim3 grid, dim3 block, cudaStream_t s) {
-    k_sweep_pair<S, Q, MK, PAT><<<grid, block, 0, s>>>(a);
-    return cudaGetLastError();
+    return launch_chained(&k_sweep_pair<S, Q, MK, PAT>, grid, block, 0, s, a);
 }
 
 template <class S, int Q, int MK>
@@ -50,8 +62,7 @@ SweepLauncher pick_pair_pattern(int pat) {
 
 template <class S, int Q, int MK, int PAT>
 cudaError_t launch_sweep_quad(const SweepArgs& a, dim3 grid, dim3 block, cudaStream_t s) {
-    k_sweep_quad<S, Q, MK, PAT><<<grid, block, 0, s>>>(a);
-    return cudaGetLastError();
+    return launch_chained(&k_sweep_quad<S, Q, MK, PAT>, grid, block, 0, s, a);
 }
 
 template <class S, int Q, int MK>
@@ -114,8 +125,7 @@ using SparseSetLauncher = cudaError_t (*)(const SparseArgs&, const double*, cons
 template <class S, class R, int Q, int MK>
 cudaError_t launch_sparse(const SparseArgs& a, cudaStream_t s) {
     const long long blocks = (a.n_fluid + 255) / 256;
-    k_sweep_sparse<S, R, Q, MK><<<(unsigned)blocks, 256, 0, s>>>(a);
-    return cudaGetLastError();
+    return launch_chained(&k_sweep_sparse<S, R, Q, MK>, dim3((unsigned)blocks), dim3(256), 0, s, a);
 }
 
 template <class S, class R, int Q, int MK>
@@ -127,16 +137,14 @@ cudaError_t launch_sparse_set(const SparseArgs& a, const double* rho, const doub
 
 template <class S, class R, int Q, int MK, int PAT>
 cudaError_t launch_sweep_zpipe(const SweepArgs& a, dim3 grid, dim3 block, cudaStream_t s) {
-    k_sweep_zpipe<S, R, Q, MK, PAT><<<grid, block, 0, s>>>(a);
-    return cudaGetLastError();
+    return launch_chained(&k_sweep_zpipe<S, R, Q, MK, PAT>, grid, block, 0, s, a);
 }
 
 using BatchLauncher = cudaError_t (*)(const BatchArgs&, dim3, dim3, cudaStream_t);
 
 template <class S, class R, int Q, int MK, int PAT>
 cudaError_t launch_batched(const BatchArgs& b, dim3 grid, dim3 block, cudaStream_t s) {
-    k_sweep_batched<S, R, Q, MK, PAT><<<grid, block, 0, s>>>(b);
-    return cudaGetLastError();
+    return launch_chained(&k_sweep_batched<S, R, Q, MK, PAT>, grid, block, 0, s, b);
 }
 
 template <class S, class R, int Q, int MK>
@@ -178,8 +186,7 @@ SweepLauncher pick_sweep_pattern(int pat) {
 
 template <class S, class R, int Q, int MK, int PAT>
 cudaError_t launch_prepass(const SweepArgs& a, dim3 grid, dim3 block, cudaStream_t s) {
-    k_boundary_prepass<S, R, Q, MK, PAT><<<grid, block, 0, s>>>(a);
-    return cudaGetLastError();
+    return launch_chained(&k_boundary_prepass<S, R, Q, MK, PAT>, grid, block, 0, s, a);
 }
 
 template <class S, class R, int Q, int MK>

@@ -355,6 +355,7 @@ template <> struct SweepMinBlocks<float, 27, MK_MRT, PAT_PULL> { static constexp
 // WALLS false: for domains without flags.
 template <class S, class R, int Q, int MK, int PAT, bool WALLS = true>
 __global__ void __launch_bounds__(256, SweepMinBlocks<S, Q, MK, PAT>::value) k_sweep(const SweepArgs a) {
+    chain_wait();
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     const int y = blockIdx.y * blockDim.y + threadIdx.y;
     const int z = blockIdx.z;
@@ -369,6 +370,7 @@ __global__ void __launch_bounds__(256, SweepMinBlocks<S, Q, MK, PAT>::value) k_s
 // cell reads and the locations it writes are the same set, disjoint from every other cell's.
 template <class S, class R, int Q, int MK, int PAT>
 __global__ void __launch_bounds__(256, 2) k_sweep_zpipe(const SweepArgs a) {
+    chain_wait();
     static_assert(PAT == PAT_PULL || PAT == PAT_AA_EVEN || PAT == PAT_AA_ODD, "pipelined sweep: pull and AA");
     using A = Access<PAT>;
     const Grid& g = a.g;
@@ -439,6 +441,7 @@ __device__ __forceinline__ void prefetch_cell(const SweepArgs& a, int x, int y, 
 // registers, so they are summed here first, for every pattern.
 template <class S, class R, int Q, int PAT>
 __global__ void __launch_bounds__(256) k_ubb_density(const SweepArgs a, R* rho_out) {
+    chain_wait();
     using L = Lat<Q>;
     using PA = Access<PrevPattern<PAT>::value>;
     const Grid& g = a.g;
@@ -493,6 +496,7 @@ template <class S, int Q, int MK> struct BatchMinBlocks { static constexpr int v
 
 template <class S, class R, int Q, int MK, int PAT>
 __global__ void __launch_bounds__(256, BatchMinBlocks<S, Q, MK>::value) k_sweep_batched(const BatchArgs b) {
+    chain_wait();
     __shared__ __align__(16) SweepArgs sa;
     constexpr int WORDS = sizeof(SweepArgs) / 4;
     static_assert(sizeof(SweepArgs) % 4 == 0, "SweepArgs is copied as 32-bit words");
@@ -537,6 +541,7 @@ struct SparseArgs {
 
 template <class S, class R, int Q, int MK>
 __global__ void __launch_bounds__(256) k_sweep_sparse(const SparseArgs a) {
+    chain_wait();
     const long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (c >= a.n_fluid) return;
     const S* src = static_cast<const S*>(a.src);
@@ -577,6 +582,7 @@ __global__ void __launch_bounds__(256) k_sparse_set_equilibrium(const SparseArgs
 template <class S, class R, int Q>
 __global__ void __launch_bounds__(256) k_sparse_ubb(const SparseArgs a, const unsigned* links, long long n_links,
                                                     double ux, double uy, double uz) {
+    chain_wait();
     using L = Lat<Q>;
     const long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (k >= n_links) return;
@@ -682,6 +688,7 @@ __global__ void __launch_bounds__(256) k_set_equilibrium(const MacroArgs a) {
 // A link whose table is missing, or whose other cell lies beyond the ghost layer, gets NoSlip.
 template <class S, class R, int Q, int MK, int PAT>
 __global__ void __launch_bounds__(256) k_boundary_prepass(const SweepArgs a) {
+    chain_wait();
     using L = Lat<Q>;
     using A = Access<PAT>;
     using PA = Access<PrevPattern<PAT>::value>;

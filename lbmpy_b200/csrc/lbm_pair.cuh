@@ -108,6 +108,7 @@ __global__ void __launch_bounds__(32 * PAIR_ROWS, PairMinBlocks<S>::value) k_swe
     using A = Access<PAT>;
     using PS = Pair<S>;
     constexpr int ADDR = AddrOf<MK>::value;
+    chain_wait();
     const Grid& g = a.g;
     const int lane = threadIdx.x;
     const int pairs_per_row = g.nx >> 1;

@@ -47,6 +47,7 @@ __global__ void __launch_bounds__(256, 3) k_sweep_closure_tc(const SweepArgs a) 
     using A = Access<PAT>;
     __shared__ MlpShared sp;
     __shared__ __align__(16) uint32_t tiles[8][32 * MLP_XLD];
+    chain_wait();
     const int tid = threadIdx.x + threadIdx.y * blockDim.x;
     static_assert(sizeof(MlpShared) % 16 == 0, "the image is copied in 16-byte pieces");
     for (int i = tid; i < int(sizeof(MlpShared) / 16); i += blockDim.x * blockDim.y)
@@ -95,8 +96,7 @@ __global__ void __launch_bounds__(256, 3) k_sweep_closure_tc(const SweepArgs a) 
 template <int PAT>
 cudaError_t launch_closure_tc(const SweepArgs& a, dim3 grid, dim3 block, cudaStream_t s) {
     if (block.x * block.y != 256) return cudaErrorInvalidConfiguration;
-    k_sweep_closure_tc<PAT><<<grid, block, 0, s>>>(a);
-    return cudaGetLastError();
+    return launch_chained(&k_sweep_closure_tc<PAT>, grid, block, 0, s, a);
 }
 
 SweepLauncher sweep_q27_closure(int store, int pat) {

@@ -59,6 +59,7 @@ __global__ void __launch_bounds__(32 * QUAD_ROWS, 4) k_sweep_quad(const SweepArg
     using L = Lat<Q>;
     using A = Access<PAT>;
     constexpr int ADDR = AddrOf<MK>::value;
+    chain_wait();
     const Grid& g = a.g;
     const int lane = threadIdx.x;
     const int quads_per_row = g.nx >> 2;

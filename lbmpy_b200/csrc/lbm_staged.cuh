@@ -128,6 +128,7 @@ __device__ __forceinline__ void staged_warp_dispatch(int warp, F&& f) {
 // byte 248), then the stages.
 template <class S, class R, int Q, int MK, int PAT, int W>
 __global__ void __launch_bounds__(W) k_sweep_staged(const SweepArgs a, const int ns) {
+    chain_wait();
     static_assert(PAT == PAT_PULL || PAT == PAT_AA_EVEN || PAT == PAT_AA_ODD, "staged sweep: pull and AA");
     static_assert(W % 32 == 0 && W >= 32 && W <= 1024, "staged sweep: whole warps");
     using A = Access<PAT>;
