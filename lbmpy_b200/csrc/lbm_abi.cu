@@ -950,7 +950,16 @@ static int macro_common(const LbmPlan* p, const void* pdfs, const int64_t stride
     a.u = const_cast<void*>(u);
     for (int k = 0; k < 3; ++k) a.rs[k] = rho ? rs[k] : 0;
     for (int k = 0; k < 4; ++k) a.us[k] = u ? us[k] : 0;
+    a.staged = (rho == nullptr || rs[2] == 1) && (u == nullptr || (us[3] == 1 && us[2] == 3)) &&
+               (rho != nullptr || u != nullptr) && a.g.ny <= 65535;
     return LBM_OK;
+}
+
+// Launch shape of the getter and the setter.
+static void macro_shape(const MacroArgs& a, dim3& grid, dim3& block) {
+    if (!a.staged) return launch_shape(a.g, 1, grid, block);
+    block = dim3(MACRO_X, 1, MACRO_Z);
+    grid = dim3((a.g.nx + MACRO_X - 1) / MACRO_X, a.g.ny, (a.g.nz + MACRO_Z - 1) / MACRO_Z);
 }
 
 int lbm_set_equilibrium(const LbmPlan* p, void* pdfs, const int64_t strides[4], const void* rho,
@@ -964,7 +973,7 @@ int lbm_set_equilibrium(const LbmPlan* p, void* pdfs, const int64_t strides[4], 
     MacroLauncher L = set_eq_launcher(p, pattern_kind(p, prev_parity ? 1 : 0));
     if (L == nullptr) return fail(LBM_E_UNSUPPORTED, "no setter kernel");
     dim3 grid, block;
-    launch_shape(a.g, 1, grid, block);
+    macro_shape(a, grid, block);
     cudaError_t e = L(a, grid, block, static_cast<cudaStream_t>(stream));
     return e == cudaSuccess ? LBM_OK : cuda_fail(e, "setter launch");
 }
@@ -980,7 +989,7 @@ int lbm_get_macroscopic(const LbmPlan* p, const void* pdfs, const int64_t stride
     MacroLauncher L = p->q == 19 ? get_launcher_q<19>(p->store, pat) : get_launcher_q<27>(p->store, pat);
     if (L == nullptr) return fail(LBM_E_UNSUPPORTED, "no getter kernel");
     dim3 grid, block;
-    launch_shape(a.g, 1, grid, block);
+    macro_shape(a, grid, block);
     cudaError_t e = L(a, grid, block, static_cast<cudaStream_t>(stream));
     return e == cudaSuccess ? LBM_OK : cuda_fail(e, "getter launch");
 }

@@ -633,6 +633,31 @@ struct MacroArgs {
     void* u;                // R*, element strides us[4] (x, y, z, component)
     long long rs[3];
     long long us[4];
+    int staged;             // rho and u are C-ordered: z fastest, then (for u behind its component) z
+};
+
+// C-ordered macroscopic fields (numpy's and torch's default) run along z while the populations run along x:
+// thread by thread every 4-byte access would touch its own 32-byte sector.  Blocks of 32 x 8 cells in x and
+// z pass them through shared memory instead, in whole sectors.
+constexpr int MACRO_X = 32, MACRO_Z = 8;
+template <class R> struct MacroTile {
+    R rho[MACRO_X][MACRO_Z + 1];
+    R u[MACRO_X][3 * MACRO_Z + 1];
+    // Calls op(shared element, element index) for every element of the block's part of rho or u.
+    template <class F> __device__ __forceinline__ void each_rho(const MacroArgs& a, int x0, int y, int z0, F op) {
+        const int tid = threadIdx.x + MACRO_X * threadIdx.z;
+        const int x = tid / MACRO_Z, z = tid % MACRO_Z;
+        if (x0 + x < a.g.nx && z0 + z < a.g.nz) op(rho[x][z], (x0 + x) * a.rs[0] + y * a.rs[1] + (z0 + z));
+    }
+    template <class F> __device__ __forceinline__ void each_u(const MacroArgs& a, int x0, int y, int z0, F op) {
+        const int tid = threadIdx.x + MACRO_X * threadIdx.z;
+#pragma unroll
+        for (int e = tid; e < MACRO_X * MACRO_Z * 3; e += MACRO_X * MACRO_Z) {
+            const int x = e / (3 * MACRO_Z), k = e % (3 * MACRO_Z);
+            if (x0 + x < a.g.nx && z0 + k / 3 < a.g.nz)
+                op(u[x][k], (x0 + x) * a.us[0] + y * a.us[1] + 3LL * z0 + k);
+        }
+    }
 };
 
 // Equilibrium initialisation through the write accessor of the previous step
@@ -644,13 +669,26 @@ __global__ void __launch_bounds__(256) k_set_equilibrium(const MacroArgs a) {
     const Grid& g = a.g;
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     const int y = blockIdx.y * blockDim.y + threadIdx.y;
-    const int z = blockIdx.z;
-    if (x >= g.nx || y >= g.ny) return;
+    const int z = blockIdx.z * blockDim.z + threadIdx.z;
     const R* rp = static_cast<const R*>(a.rho);
     const R* up = static_cast<const R*>(a.u);
-    const R rho = rp[x * a.rs[0] + y * a.rs[1] + z * a.rs[2]];
-    const long long ub = x * a.us[0] + y * a.us[1] + z * a.us[2];
-    R ux = up[ub], uy = up[ub + a.us[3]], uz = up[ub + 2 * a.us[3]];
+    R rho, ux, uy, uz;
+    if (a.staged) {
+        __shared__ MacroTile<R> tile;
+        const int x0 = blockIdx.x * MACRO_X, z0 = blockIdx.z * MACRO_Z;
+        tile.each_rho(a, x0, y, z0, [&](R& v, long long e) { v = rp[e]; });
+        tile.each_u(a, x0, y, z0, [&](R& v, long long e) { v = up[e]; });
+        __syncthreads();
+        if (x >= g.nx || z >= g.nz) return;
+        rho = tile.rho[threadIdx.x][threadIdx.z];
+        const R* u = &tile.u[threadIdx.x][3 * threadIdx.z];
+        ux = u[0]; uy = u[1]; uz = u[2];
+    } else {
+        if (x >= g.nx || y >= g.ny) return;
+        rho = rp[x * a.rs[0] + y * a.rs[1] + z * a.rs[2]];
+        const long long ub = x * a.us[0] + y * a.us[1] + z * a.us[2];
+        ux = up[ub]; uy = up[ub + a.us[3]]; uz = up[ub + 2 * a.us[3]];
+    }
     if (a.p.force_model != FM_NONE) {
         const R h = R(0.5) / (a.p.compressible ? rho : R(1));
         ux -= h * R(a.p.force[0]); uy -= h * R(a.p.force[1]); uz -= h * R(a.p.force[2]);
@@ -804,25 +842,40 @@ __global__ void __launch_bounds__(256) k_get_macroscopic(const MacroArgs a) {
     const Grid& g = a.g;
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     const int y = blockIdx.y * blockDim.y + threadIdx.y;
-    const int z = blockIdx.z;
-    if (x >= g.nx || y >= g.ny) return;
-    NbrOffsets nb;
-    nb.init(g, x, y, z);
-    const int cell = (x + 1) + (y + 1) * g.sy + (z + 1) * g.sz;
-    const S* src = static_cast<const S*>(a.pdfs);
-    R f[Q];
-#pragma unroll
-    for (int i = 0; i < Q; ++i) {
-        const int off = nb.off(A::template woff<Q>(i, 0), A::template woff<Q>(i, 1), A::template woff<Q>(i, 2));
-        f[i] = Conv<S, R>::ld(at(src, A::template wslot<Q>(i) * g.sq, cell + off));
-    }
-    Macro<Q, R> m = conserved<Q, R>(f, a.p, false);
-    if (a.p.force_model != FM_NONE) {
-        const R h = R(0.5) / m.rho_ref;
-        m.ux += h * R(a.p.force[0]); m.uy += h * R(a.p.force[1]); m.uz += h * R(a.p.force[2]);
-    }
+    const int z = blockIdx.z * blockDim.z + threadIdx.z;
+    const bool inside = x < g.nx && y < g.ny && z < g.nz;
+    if (!inside && !a.staged) return;
     R* rp = static_cast<R*>(a.rho);
     R* up = static_cast<R*>(a.u);
+    Macro<Q, R> m{};
+    if (inside) {
+        NbrOffsets nb;
+        nb.init(g, x, y, z);
+        const int cell = (x + 1) + (y + 1) * g.sy + (z + 1) * g.sz;
+        const S* src = static_cast<const S*>(a.pdfs);
+        R f[Q];
+#pragma unroll
+        for (int i = 0; i < Q; ++i) {
+            const int off = nb.off(A::template woff<Q>(i, 0), A::template woff<Q>(i, 1), A::template woff<Q>(i, 2));
+            f[i] = Conv<S, R>::ld(at(src, A::template wslot<Q>(i) * g.sq, cell + off));
+        }
+        m = conserved<Q, R>(f, a.p, false);
+        if (a.p.force_model != FM_NONE) {
+            const R h = R(0.5) / m.rho_ref;
+            m.ux += h * R(a.p.force[0]); m.uy += h * R(a.p.force[1]); m.uz += h * R(a.p.force[2]);
+        }
+    }
+    if (a.staged) {
+        __shared__ MacroTile<R> tile;
+        const int x0 = blockIdx.x * MACRO_X, z0 = blockIdx.z * MACRO_Z;
+        tile.rho[threadIdx.x][threadIdx.z] = m.rho;
+        R* u = &tile.u[threadIdx.x][3 * threadIdx.z];
+        u[0] = m.ux; u[1] = m.uy; u[2] = m.uz;
+        __syncthreads();
+        if (rp) tile.each_rho(a, x0, y, z0, [&](R& v, long long e) { rp[e] = v; });
+        if (up) tile.each_u(a, x0, y, z0, [&](R& v, long long e) { up[e] = v; });
+        return;
+    }
     if (rp) rp[x * a.rs[0] + y * a.rs[1] + z * a.rs[2]] = m.rho;
     if (up) {
         const long long ub = x * a.us[0] + y * a.us[1] + z * a.us[2];
