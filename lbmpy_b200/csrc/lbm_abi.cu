@@ -16,6 +16,7 @@
 #include "../../include/lbm_b200.h"
 #include "lbm_closure.cuh"
 #include "lbm_dispatch.h"
+#include "lbm_mrt1.h"
 #include "lbm_reduce.cuh"
 
 using namespace lbm;
@@ -165,6 +166,7 @@ SweepLauncher sweep_launcher(const LbmPlan* p, int pat) {
     if (p->q == 19 && p->mk == MK_MRT) return sweep_q19_mrt(p->store, pat);
     if (p->q == 27 && p->mk == MK_POP) return sweep_q27_pop(p->store, pat);
     if (p->q == 27 && p->mk == MK_MRT) return sweep_q27_mrt(p->store, pat);
+    if (p->mk == MK_MRT1) return p->q == 19 ? sweep_q19_mrt1(p->store, pat) : sweep_q27_mrt1(p->store, pat);
     if (p->q == 27 && p->mk == MK_CUM) return sweep_q27_cum(p->store, pat);
     if (p->q == 27 && p->mk == MK_CUM1) return sweep_q27_cum1(p->store, pat);
     if (p->q == 27 && p->mk == MK_CUM1_MLP) return sweep_q27_closure(p->store, pat);
@@ -177,6 +179,7 @@ SweepLauncher pair_launcher(const LbmPlan* p, int pat) {
     if (p->q == 19 && p->mk == MK_MRT) return sweep_pair_q19_mrt(p->store, pat);
     if (p->q == 27 && p->mk == MK_POP) return sweep_pair_q27_pop(p->store, pat);
     if (p->q == 27 && p->mk == MK_MRT) return sweep_pair_q27_mrt(p->store, pat);
+    if (p->mk == MK_MRT1) return p->q == 19 ? sweep_pair_q19_mrt1(p->store, pat) : sweep_pair_q27_mrt1(p->store, pat);
     if (p->q == 27 && p->mk == MK_CUM) return sweep_pair_q27_cum(p->store, pat);
     if (p->q == 27 && p->mk == MK_CUM1) return sweep_pair_q27_cum1(p->store, pat);
     return nullptr;
@@ -192,6 +195,7 @@ SweepLauncher quad_launcher(const LbmPlan* p, int pat) {
     if (p->q == 19 && p->mk == MK_POP) return sweep_quad_q19_pop(p->store, pat);
     if (p->q == 19 && p->mk == MK_MRT) return sweep_quad_q19_mrt(p->store, pat);
     if (p->q == 27 && p->mk == MK_POP) return sweep_quad_q27_pop(p->store, pat);
+    if (p->q == 19 && p->mk == MK_MRT1) return sweep_quad_q19_mrt1(p->store, pat);
     if (p->q == 27 && p->mk == MK_CUM) return sweep_quad_q27_cum(p->store, pat);
     if (p->q == 27 && p->mk == MK_CUM1) return sweep_quad_q27_cum1(p->store, pat);
     return nullptr;
@@ -241,9 +245,9 @@ bool pair_applicable(const LbmPlan* p, const void* src, const void* dst, const i
 
 SweepLauncher prepass_launcher(const LbmPlan* p, int pat) {
     if (p->q == 19 && p->mk == MK_POP) return prepass_q19_pop(p->store, pat);
-    if (p->q == 19 && p->mk == MK_MRT) return prepass_q19_mrt(p->store, pat);
+    if (p->q == 19 && (p->mk == MK_MRT || p->mk == MK_MRT1)) return prepass_q19_mrt(p->store, pat);
     if (p->q == 27 && p->mk == MK_POP) return prepass_q27_pop(p->store, pat);
-    if (p->q == 27 && p->mk == MK_MRT) return prepass_q27_mrt(p->store, pat);
+    if (p->q == 27 && (p->mk == MK_MRT || p->mk == MK_MRT1)) return prepass_q27_mrt(p->store, pat);
     if (p->q == 27 && p->mk == MK_CUM) return prepass_q27_cum(p->store, pat);
     if (p->q == 27 && (p->mk == MK_CUM1 || p->mk == MK_CUM1_MLP)) return prepass_q27_cum1(p->store, pat);
     if (p->q == 27 && p->mk == MK_CM) return prepass_q27_cm(p->store, pat);
@@ -252,9 +256,9 @@ SweepLauncher prepass_launcher(const LbmPlan* p, int pat) {
 
 StagedLauncher staged_launcher(const LbmPlan* p, int pat) {
     if (p->q == 19 && p->mk == MK_POP) return sweep_staged_q19_pop(p->store, pat);
-    if (p->q == 19 && p->mk == MK_MRT) return sweep_staged_q19_mrt(p->store, pat);
+    if (p->q == 19 && (p->mk == MK_MRT || p->mk == MK_MRT1)) return sweep_staged_q19_mrt(p->store, pat);
     if (p->q == 27 && p->mk == MK_POP) return sweep_staged_q27_pop(p->store, pat);
-    if (p->q == 27 && p->mk == MK_MRT) return sweep_staged_q27_mrt(p->store, pat);
+    if (p->q == 27 && (p->mk == MK_MRT || p->mk == MK_MRT1)) return sweep_staged_q27_mrt(p->store, pat);
     if (p->q == 27 && p->mk == MK_CUM) return sweep_staged_q27_cum(p->store, pat);
     if (p->q == 27 && p->mk == MK_CUM1) return sweep_staged_q27_cum1(p->store, pat);
     return nullptr;
@@ -280,9 +284,9 @@ bool staged_applicable(const LbmPlan* p, const void* src, const int64_t s[4], in
 
 MacroLauncher set_eq_launcher(const LbmPlan* p, int pat) {
     if (p->q == 19 && p->mk == MK_POP) return set_eq_q19_pop(p->store, pat);
-    if (p->q == 19 && p->mk == MK_MRT) return set_eq_q19_mrt(p->store, pat);
+    if (p->q == 19 && (p->mk == MK_MRT || p->mk == MK_MRT1)) return set_eq_q19_mrt(p->store, pat);
     if (p->q == 27 && p->mk == MK_POP) return set_eq_q27_pop(p->store, pat);
-    if (p->q == 27 && p->mk == MK_MRT) return set_eq_q27_mrt(p->store, pat);
+    if (p->q == 27 && (p->mk == MK_MRT || p->mk == MK_MRT1)) return set_eq_q27_mrt(p->store, pat);
     if (p->q == 27 && (p->mk == MK_CUM || p->mk == MK_CUM1 || p->mk == MK_CUM1_MLP))
         return set_eq_q27_cum(p->store, pat);
     if (p->q == 27 && p->mk == MK_CM) return set_eq_q27_cm(p->store, pat);
@@ -579,8 +583,27 @@ bool cumulant_high_orders_relax_to_equilibrium(const LbmPlanDesc* d) {
     return true;
 }
 
+// Every MRT moment of order >= 3 (indices 10 and up in both bases) has rate 1, the shear moments (4-8)
+// share one rate, a subgrid-scale model adapts none of the former and all or none of the latter, and
+// with a force the conserved moments have rate 0: the sweep that keeps only the second-order
+// non-equilibrium (collide_mrt1) gives the same state with half the arithmetic.
+bool mrt_high_orders_relax_to_equilibrium(const LbmPlanDesc* d) {
+    for (int k = 10; k < d->stencil; ++k) {
+        if (d->rates[k] != 1.0) return false;
+        if (d->sgs != LBM_SGS_NONE && ((d->sgs_mask >> k) & 1u)) return false;
+    }
+    for (int k = 5; k < 9; ++k) {
+        if (d->rates[k] != d->rates[4]) return false;
+        if (d->sgs != LBM_SGS_NONE && ((d->sgs_mask >> k) & 1u) != ((d->sgs_mask >> 4) & 1u)) return false;
+    }
+    if (d->force_model != LBM_FORCE_NONE)
+        for (int k = 0; k < 4; ++k)
+            if (d->rates[k] != 0.0 || (d->sgs != LBM_SGS_NONE && ((d->sgs_mask >> k) & 1u))) return false;
+    return true;
+}
+
 int method_kind(const LbmPlanDesc* d) {
-    if (d->method == LBM_METHOD_MRT) return MK_MRT;
+    if (d->method == LBM_METHOD_MRT) return mrt_high_orders_relax_to_equilibrium(d) ? MK_MRT1 : MK_MRT;
     if (d->method == LBM_METHOD_CENTRAL_MOMENT) return MK_CM;
     if (d->method != LBM_METHOD_CUMULANT) return MK_POP;
     if (d->fourth_order_limiter > 0.0 || !cumulant_high_orders_relax_to_equilibrium(d)) return MK_CUM;
@@ -1115,6 +1138,7 @@ SparseLauncher sparse_launcher(const LbmPlan* p) {
     if (p->q == 19 && p->mk == MK_MRT) return sparse_q19_mrt(p->store);
     if (p->q == 27 && p->mk == MK_POP) return sparse_q27_pop(p->store);
     if (p->q == 27 && p->mk == MK_MRT) return sparse_q27_mrt(p->store);
+    if (p->mk == MK_MRT1) return p->q == 19 ? sparse_q19_mrt1(p->store) : sparse_q27_mrt1(p->store);
     if (p->q == 27 && p->mk == MK_CUM) return sparse_q27_cum(p->store);
     if (p->q == 27 && p->mk == MK_CUM1) return sparse_q27_cum1(p->store);
     if (p->q == 27 && p->mk == MK_CM) return sparse_q27_cm(p->store);
@@ -1123,9 +1147,9 @@ SparseLauncher sparse_launcher(const LbmPlan* p) {
 
 SparseSetLauncher sparse_set_launcher(const LbmPlan* p) {
     if (p->q == 19 && p->mk == MK_POP) return sparse_set_q19_pop(p->store);
-    if (p->q == 19 && p->mk == MK_MRT) return sparse_set_q19_mrt(p->store);
+    if (p->q == 19 && (p->mk == MK_MRT || p->mk == MK_MRT1)) return sparse_set_q19_mrt(p->store);
     if (p->q == 27 && p->mk == MK_POP) return sparse_set_q27_pop(p->store);
-    if (p->q == 27 && p->mk == MK_MRT) return sparse_set_q27_mrt(p->store);
+    if (p->q == 27 && (p->mk == MK_MRT || p->mk == MK_MRT1)) return sparse_set_q27_mrt(p->store);
     if (p->q == 27 && (p->mk == MK_CUM || p->mk == MK_CUM1)) return sparse_set_q27_cum(p->store);
     if (p->q == 27 && p->mk == MK_CM) return sparse_set_q27_cm(p->store);
     return nullptr;
@@ -1267,6 +1291,7 @@ BatchLauncher batched_launcher(int q, int mk, int store, int pat) {
     if (q == 19 && mk == MK_MRT) return batched_q19_mrt(store, pat);
     if (q == 27 && mk == MK_POP) return batched_q27_pop(store, pat);
     if (q == 27 && mk == MK_MRT) return batched_q27_mrt(store, pat);
+    if (mk == MK_MRT1) return q == 19 ? batched_q19_mrt1(store, pat) : batched_q27_mrt1(store, pat);
     if (q == 27 && mk == MK_CUM) return batched_q27_cum(store, pat);
     if (q == 27 && mk == MK_CUM1) return batched_q27_cum1(store, pat);
     if (q == 27 && mk == MK_CM) return batched_q27_cm(store, pat);
@@ -1345,7 +1370,7 @@ int lbm_batch_create(const LbmPlanDesc* common, const LbmDomainDesc* domains, in
     if ((rc = check_device_ptr(&p0, flags, "flags", true))) return rc;
 
     // Every domain on its own, then the batch as a whole.
-    bool all_cum1 = true;
+    bool all_cum1 = true, all_mrt1 = true;
     std::vector<std::pair<int64_t, int64_t>> fields, flag_ranges;
     int64_t cells = 0;
     for (int k = 0; k < n_domains; ++k) {
@@ -1368,6 +1393,7 @@ int lbm_batch_create(const LbmPlanDesc* common, const LbmDomainDesc* domains, in
             return fail(LBM_E_INVALID, "domain %d: flags_offset must be >= 0 or -1", k);
         }
         if (!cumulant_high_orders_relax_to_equilibrium(&pk.desc)) all_cum1 = false;
+        if (!mrt_high_orders_relax_to_equilibrium(&pk.desc)) all_mrt1 = false;
         if (needs_ubb_density(&pk.desc, 0) && d.flags_offset >= 0)
             return fail(LBM_E_UNSUPPORTED, "domain %d: moving UBB walls of a compressible method are not built "
                         "for batches", k);
@@ -1382,6 +1408,7 @@ int lbm_batch_create(const LbmPlanDesc* common, const LbmDomainDesc* domains, in
              : common->method == LBM_METHOD_CUMULANT ? MK_CUM
              : common->method == LBM_METHOD_CENTRAL_MOMENT ? MK_CM : MK_POP;
     if (mk == MK_CUM && all_cum1) mk = MK_CUM1;
+    if (mk == MK_MRT && all_mrt1) mk = MK_MRT1;
     const int store = common->store_dtype;
     if (batched_launcher(q, mk, store, PAT_PULL) == nullptr)
         return fail(LBM_E_UNSUPPORTED, "no batched kernel for this stencil/method/dtype");
