@@ -26,7 +26,7 @@ struct LbmPlan {
     int device;
     int q, mk, store;
     int use_pair;          // -1 default policy, 0 never, 1 whenever applicable (environment LBM_B200_PAIR)
-    int zc;                // z-planes per thread of the FP32 closure sweep (environment LBM_B200_ZC, else 8)
+    int zc;                // z-planes per thread of the FP32 closure sweep (environment LBM_B200_ZC, else 4)
     int use_quad;          // -1 default policy, 0 never, 1 whenever applicable (environment LBM_B200_QUAD)
     int use_staged;        // -1 default policy, 0 never, 1 whenever applicable (environment LBM_B200_STAGED)
     int ns;                // shared-memory stages of the staged sweep (environment LBM_B200_NS, else 2)
@@ -719,7 +719,7 @@ int lbm_plan_create(const LbmPlanDesc* desc, LbmPlan** out) {
         const char* qenv = getenv("LBM_B200_QUAD");
         p->use_quad = qenv == nullptr ? -1 : (qenv[0] == '0' ? 0 : 1);
         const char* zenv = getenv("LBM_B200_ZC");
-        p->zc = zenv != nullptr ? atoi(zenv) : 8;
+        p->zc = zenv != nullptr ? atoi(zenv) : 4;
         if (p->zc < 1) p->zc = 1;
         const char* senv = getenv("LBM_B200_STAGED");
         p->use_staged = senv == nullptr ? -1 : (senv[0] == '0' ? 0 : 1);

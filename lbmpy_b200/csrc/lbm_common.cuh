@@ -237,7 +237,7 @@ struct SweepArgs {
     const void* src;
     void* dst;
     float* omega_out;      // optional per-cell effective shear rate (interior, x fastest)
-    int zc;                // closure sweep: consecutive z-planes per thread (next plane prefetched to L2)
+    int zc;                // closure sweep: consecutive z-planes per thread
     int stage_probe;       // staged sweep: before its last tile each CTA also waits on a barrier that
                            // nothing arrives at (exercises the bounded wait and the status report)
     unsigned long long stage_wait_ns;   // staged sweep: bound of each barrier wait (0: 1 s)

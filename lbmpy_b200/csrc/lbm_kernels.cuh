@@ -416,24 +416,6 @@ __global__ void __launch_bounds__(256, 2) k_sweep_zpipe(const SweepArgs a) {
     }
 }
 
-// Asks L2 for the lines one cell will pull (prefetch.global.L2 is a hint: no data returns, no
-// registers are held, and every address is one the sweep itself reads).
-template <class S, int Q, int PAT>
-__device__ __forceinline__ void prefetch_cell(const SweepArgs& a, int x, int y, int z) {
-    using A = Access<PAT>;
-    const Grid& g = a.g;
-    NbrOffsets nb;
-    nb.init(g, x, y, z);
-    const int cell = (x + 1) + (y + 1) * g.sy + (z + 1) * g.sz;
-    const S* src = static_cast<const S*>(a.src);
-#pragma unroll
-    for (int i = 0; i < Q; ++i) {
-        const int off = nb.off(A::template roff<Q>(i, 0), A::template roff<Q>(i, 1), A::template roff<Q>(i, 2));
-        const S* q = at(src, A::template rslot<Q>(i) * g.sq, cell + off);
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(q));
-    }
-}
-
 // Density, at the previous step, of every fluid cell with a moving-wall (UBB) link, for the
 // compressible UBB: lbmpy takes it from the cell's own post-collision values in a boundary pass
 // before the sweep (boundaries/boundaryconditions.py:794-841).  Inside an in-place sweep the

@@ -40,10 +40,15 @@ struct WarpClosureNu {
 
 // FP32 closure sweep.  The network works on whole warps, so no lane leaves early: lanes past the
 // row end work on a clamped copy of the last cell and boundary cells collide their own (unused)
-// values; only fluid cells inside the domain store.  Each thread sweeps a.zc consecutive planes
-// (amortising the parameter staging) and prefetches the next plane to L2.  Otherwise as k_sweep.
+// values; only fluid cells inside the domain store.  Otherwise as k_sweep.
+//
+// Bound by instruction issue.  Each thread sweeps a.zc consecutive planes, which amortises staging the
+// parameters; 4 blocks per SM (64 registers, 20 bytes spilled) and no prefetch of the next plane (27
+// addresses a cell) leave the least to issue and the most warps to hide the rest.  AA, periodic, on
+// B200: 128^3 127 us with 3 blocks, 8 planes and the prefetch, 120 us so (4 blocks: 1 plane 124, 2 planes
+// 122, 8 planes 124 us); 256x128x128 246 -> 230 us.
 template <int PAT>
-__global__ void __launch_bounds__(256, 3) k_sweep_closure_tc(const SweepArgs a) {
+__global__ void __launch_bounds__(256, 4) k_sweep_closure_tc(const SweepArgs a) {
     using A = Access<PAT>;
     __shared__ MlpShared sp;
     __shared__ __align__(16) uint32_t tiles[8][32 * MLP_XLD];
@@ -65,7 +70,6 @@ __global__ void __launch_bounds__(256, 3) k_sweep_closure_tc(const SweepArgs a) 
     float* dst = static_cast<float*>(a.dst);
 #pragma unroll 1
     for (int z = z0; z < z1; ++z) {
-        if (z + 1 < z1) prefetch_cell<float, 27, PAT>(a, x, y, z + 1);
         WallProbe<27> probe;
         probe.begin(g, x, y, z);
         NbrOffsets nb;
