@@ -83,22 +83,16 @@ __device__ __forceinline__ R smagorinsky_rate(const R (&f)[Q], const Macro<Q, R>
 }
 
 // ------------------------------------------------------------------ SRT / TRT
-template <int Q, class R, class P>
-__device__ __forceinline__ R collide_pop(R (&f)[Q], const P& p) {
+// Relaxation of every (i, inverse) pair, with the force if there is one.  PLAIN: continuous Maxwellian
+// equilibrium and no force, known at compile time.
+template <bool PLAIN, int Q, class R, class P>
+__device__ __forceinline__ void relax_pop(R (&f)[Q], const Macro<Q, R>& m, R wp, R wm, const P& p) {
     using L = Lat<Q>;
-    const bool shift = p.force_model == FM_GUO || p.force_model == FM_CENTRAL;
-    const Macro<Q, R> m = conserved<Q, R>(f, p, shift);
-    R wp = p_rate<R>(p, 0), wm = p_rate<R>(p, 1);
-    if (p.sgs == 1) {
-        const R om = smagorinsky_rate<Q, R>(f, m, p);
-        if (p.sgs_mask & 1u) wp = om;
-        if (p.sgs_mask & 2u) wm = om;
-    }
     const R rf = p.compressible ? m.rho : R(1);
     const R uxx = m.ux * m.ux, uyy = m.uy * m.uy, uzz = m.uz * m.uz;
     const R uxy = m.ux * m.uy, uxz = m.ux * m.uz, uyz = m.uy * m.uz;
-    const bool cont = p.continuous_eq != 0;
-    const bool has_force = p.force_model == FM_GUO || p.force_model == FM_SIMPLE || p.force_model == FM_LUO;
+    const bool cont = PLAIN || p.continuous_eq != 0;
+    const bool has_force = !PLAIN && (p.force_model == FM_GUO || p.force_model == FM_SIMPLE || p.force_model == FM_LUO);
     const R Fx = p_force<R>(p, 0), Fy = p_force<R>(p, 1), Fz = p_force<R>(p, 2);
     const R uF = m.ux * Fx + m.uy * Fy + m.uz * Fz;
     R fe_scale = R(1), fo_scale = R(1), fe_on = R(1);
@@ -143,6 +137,30 @@ __device__ __forceinline__ R collide_pop(R (&f)[Q], const P& p) {
             f[j] = fj + de - dod;
         }
     }
+}
+
+// Whether the SRT/TRT collision is the plain one of collide_pop: continuous equilibrium, no force.
+template <class P> __device__ __forceinline__ bool pop_is_plain(const P& p) {
+    return p.continuous_eq != 0 && p.force_model == FM_NONE;
+}
+
+// Which equilibrium and whether a force is the same for every cell, but asked for per pair it keeps the
+// compiler from scheduling the pairs together.  The plain collision therefore has its own copy of the loop:
+// chosen here once per cell (D3Q19 TRT pull FP32 512^3 on B200 3.26 -> 3.21 ms), or, PLAIN, by the launch
+// (the packed sweeps, where two copies spill: see k_sweep_quad).
+template <int Q, class R, class P, bool PLAIN = false>
+__device__ __forceinline__ R collide_pop(R (&f)[Q], const P& p) {
+    const bool shift = !PLAIN && (p.force_model == FM_GUO || p.force_model == FM_CENTRAL);
+    const Macro<Q, R> m = conserved<Q, R>(f, p, shift);
+    R wp = p_rate<R>(p, 0), wm = p_rate<R>(p, 1);
+    if (p.sgs == 1) {
+        const R om = smagorinsky_rate<Q, R>(f, m, p);
+        if (p.sgs_mask & 1u) wp = om;
+        if (p.sgs_mask & 2u) wm = om;
+    }
+    constexpr bool scalar = std::is_same<R, float>::value || std::is_same<R, double>::value;
+    if (PLAIN || (scalar && pop_is_plain(p))) relax_pop<true, Q, R>(f, m, wp, wm, p);
+    else relax_pop<false, Q, R>(f, m, wp, wm, p);
     return wp;
 }
 

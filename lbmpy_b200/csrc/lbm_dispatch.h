@@ -62,6 +62,9 @@ SweepLauncher pick_pair_pattern(int pat) {
 
 template <class S, int Q, int MK, int PAT>
 cudaError_t launch_sweep_quad(const SweepArgs& a, dim3 grid, dim3 block, cudaStream_t s) {
+    if constexpr (MK == MK_POP)
+        if (a.g.flags == nullptr && a.p.continuous_eq != 0 && a.p.force_model == FM_NONE)
+            return launch_chained(&k_sweep_quad<S, Q, MK, PAT, true>, grid, block, 0, s, a);
     return launch_chained(&k_sweep_quad<S, Q, MK, PAT>, grid, block, 0, s, a);
 }
 
