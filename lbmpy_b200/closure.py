@@ -26,6 +26,7 @@ from __future__ import annotations
 
 import ctypes
 import math
+import threading
 from typing import Optional
 
 import numpy as np
@@ -88,6 +89,7 @@ class MLPClosure:
         self.params = params.reshape(-1).to(self.device).contiguous()
         self.version = 0
         self.history = []
+        self._workspaces, self._workspace_lock = {}, threading.Lock()
 
     # ---------------------------------------------------------------------------- parameters
     @property
@@ -126,6 +128,27 @@ class MLPClosure:
                 "lbm_mlp_forward")
         return out
 
+    _MAX_WORKSPACES = 4
+
+    def _workspace(self):
+        """The reduction workspace of loss_and_grad, kept with the closure: allocating and freeing one
+        per call waits for the device twice.  One per device, stream and thread, so that calls that may
+        overlap do not share it; the least recently used is given back when there are more than a few."""
+        key = (torch.cuda.current_device(), torch.cuda.current_stream().cuda_stream, threading.get_ident())
+        with self._workspace_lock:
+            w = self._workspaces.pop(key, None) or _Trainer()
+            self._workspaces[key] = w
+            while len(self._workspaces) > self._MAX_WORKSPACES:
+                self._workspaces.pop(next(iter(self._workspaces)))
+        return w
+
+    def __getstate__(self):          # the workspaces stay with this object: copies make their own
+        return {k: v for k, v in self.__dict__.items() if not k.startswith("_workspace")}
+
+    def __setstate__(self, state):
+        self.__dict__.update(state)
+        self._workspaces, self._workspace_lock = {}, threading.Lock()
+
     def loss_and_grad(self, feats, target, weight=None, trainer=None):
         """(loss, gradient [1442]) of the weighted mean squared nu_t error, from the GPU kernels."""
         feats = feats.to(self.device, torch.float32).contiguous()
@@ -136,9 +159,8 @@ class MLPClosure:
             inv = 1.0 / float(weight.double().sum())
         else:
             inv = 1.0 / n
-        own = trainer is None
-        if own:
-            trainer = _Trainer()
+        if trainer is None:
+            trainer = self._workspace()
         grad = torch.empty(NPARAM, dtype=torch.float32, device=self.device)
         loss = torch.empty(1, dtype=torch.float64, device=self.device)
         N.check(N.lib().lbm_mlp_loss_grad(trainer.handle, _ptr(self.params), _ptr(feats), _ptr(target), _ptr(weight),

@@ -14,6 +14,7 @@ import math
 from collections import OrderedDict
 from dataclasses import dataclass, field, replace
 from fractions import Fraction
+from functools import cached_property
 from typing import Any, Iterable, List, Optional, Tuple, Union
 
 from . import _native as N
@@ -271,17 +272,20 @@ class LbMethod:
     def relaxation_rate_dict(self):
         return OrderedDict(zip(self.moments, self.relaxation_rates))
 
+    @cached_property
+    def _shear_indices(self):
+        """Positions of the shear moments: they depend on the moment groups alone (the rates are read
+        anew by every call of shear_relaxation_rate)."""
+        flat = [p for g in self.groups for p in g]
+        return tuple(start + k for g in self.groups for start in (flat.index(g[0]),) for k, p in enumerate(g)
+                     if M.is_shear(p, self.dim))
+
     @property
     def shear_relaxation_rate(self):
-        rates = {r for g in self.groups for p, r in zip(g, self._group_rates(g)) if M.is_shear(p, self.dim)}
+        rates = {self.relaxation_rates[k] for k in self._shear_indices}
         if len(rates) != 1:
             raise ValueError(f"Shear moments are relaxed with different relaxation times: {rates}")
         return rates.pop()
-
-    def _group_rates(self, group):
-        flat = [p for g in self.groups for p in g]
-        start = flat.index(group[0])
-        return self.relaxation_rates[start:start + len(group)]
 
     def __repr__(self):
         return (f"LbMethod({self.stencil.name}, {self.kind}, compressible={self.compressible}, "

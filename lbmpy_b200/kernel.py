@@ -11,6 +11,7 @@ effective shear rate) and ``stream`` (a ``torch.cuda.Stream``).
 from __future__ import annotations
 
 import ctypes
+import functools
 from typing import Dict, Optional, Sequence
 
 import torch
@@ -59,6 +60,15 @@ def free_parameters(update_rule) -> set:
     return names
 
 
+@functools.lru_cache(maxsize=None)
+def _even_odd_positions(stencil_name: str):
+    """Positions of the first even (order > 0) and the first odd moment of the stencil's default basis."""
+    from . import methods as M
+    orders = [sum(e) for e in M.default_monomials(stencil_name)]
+    return (next(k for k, n in enumerate(orders) if n % 2 == 0 and n > 0),
+            next(k for k, n in enumerate(orders) if n % 2 == 1))
+
+
 def build_desc(update_rule, dims, periodic, params: Dict, ubb_velocities=None,
                rates_needed: bool = True, fixed_density=None, ubb_options=None) -> N.LbmPlanDesc:
     """Resolves an update rule plus parameter values into the C plan descriptor.  Plans that only
@@ -77,11 +87,8 @@ def build_desc(update_rule, dims, periodic, params: Dict, ubb_velocities=None,
     ph = None if rates_needed else 1.0
     rates = [_evaluate(r, params, ph) for r in m.relaxation_rates]
     if m.kind in ("srt", "trt"):
-        from . import methods as M
-        monos = M.default_monomials(m.stencil.name)
-        even = next(r for r, e in zip(rates, monos) if sum(e) % 2 == 0 and sum(e) > 0)
-        odd = next(r for r, e in zip(rates, monos) if sum(e) % 2 == 1)
-        native_rates = [even, odd]
+        even, odd = _even_odd_positions(m.stencil.name)
+        native_rates = [rates[even], rates[odd]]
     else:
         native_rates = rates
     for k, r in enumerate(native_rates):
