@@ -845,7 +845,9 @@ static int launch_sweep_checked(const LbmPlan* p, const void* src, void* dst, co
     a.link_code = p->link_code;
     a.link_value = p->link_value;
     if (flags != nullptr && flags == p->rowmask_flags) {
-        a.g.rowmask = p->rowmask;
+        // Not periodic in x, a domain has boundary cells at the ends of every row: the summary would only
+        // delay the wall words, which the sweeps then ask for with the populations (as batches do).
+        a.g.rowmask = p->desc.periodic[0] ? p->rowmask : nullptr;
         a.g.walls = p->walls;
     }
     if (flags != nullptr && p->ubb_rho != nullptr && needs_ubb_density(&p->desc, p->ubb_link_mask)) {
