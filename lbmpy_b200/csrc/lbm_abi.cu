@@ -143,6 +143,28 @@ void launch_shape(const Grid& g, int zc, dim3& grid, dim3& block) {
     grid = dim3((g.nx + bx - 1) / bx, (g.ny + by - 1) / by, (g.nz + zc - 1) / zc);
 }
 
+// Share of the lanes of a launch that have a cell.
+double lanes_used(const Grid& g, const dim3& grid, const dim3& block) {
+    const int warps = (int(block.x * block.y) + 31) / 32;
+    return double(g.nx) * g.ny / (double(grid.x) * grid.y * warps * 32);
+}
+
+// Blocks for kernels that take one cell per thread, whatever the block: those of launch_shape, or, for
+// rows of up to 128 cells that these leave partly idle, whole rows, as many as fit 256 threads and
+// divide ny evenly (a warp then spans two rows).  The first keep their aligned segments, so the second
+// have to use at least a tenth more of the lanes.
+void cell_shape(const Grid& g, dim3& grid, dim3& block) {
+    launch_shape(g, 1, grid, block);
+    if (g.nx > 128) return;
+    int by = std::min(256 / g.nx, g.ny);
+    const int blocks = (g.ny + by - 1) / by;
+    by = (g.ny + blocks - 1) / blocks;
+    const dim3 rows(g.nx, by, 1), cover(1, (g.ny + by - 1) / by, g.nz);
+    if (cover.y > 65535 || lanes_used(g, cover, rows) < 1.1 * lanes_used(g, grid, block)) return;
+    block = rows;
+    grid = cover;
+}
+
 // In-place patterns update one field (src == dst); pull and push use two.
 bool pattern_inplace(int pattern) {
     return pattern == LBM_PATTERN_AA || pattern == LBM_PATTERN_ESOTWIST || pattern == LBM_PATTERN_ESOPULL ||
@@ -891,7 +913,8 @@ static int launch_sweep_checked(const LbmPlan* p, const void* src, void* dst, co
         grid = dim3((a.g.nx + 63) / 64, (a.g.ny + PAIR_ROWS - 1) / PAIR_ROWS, a.g.nz);
     } else {
         L = sweep_launcher(p, pat);
-        launch_shape(a.g, a.zc, grid, block);
+        if (p->mk == MK_CUM1_MLP) launch_shape(a.g, a.zc, grid, block);
+        else cell_shape(a.g, grid, block);
         if (p->block_x > 0 && a.zc == 1) {
             block = dim3(p->block_x, 256 / p->block_x, 1);
             grid = dim3((a.g.nx + block.x - 1) / block.x, (a.g.ny + block.y - 1) / block.y, a.g.nz);
