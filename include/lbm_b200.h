@@ -206,9 +206,11 @@ int lbm_plan_set_links(LbmPlan* plan, const LbmLinkTables* tables);
 /* Sets bit 7 on every fluid cell of `flags` (device, layout above) that has a boundary
  * neighbour along the plan's stencil, honouring periodicity.  Replaces the link-list setup of
  * LatticeBoltzmannBoundaryHandling (boundaries/boundaryhandling.py:15-155).
- * It also records, in the plan, which interior rows (y, z) hold a non-zero flag; the plan's
- * sweeps given this same `flags` pointer skip the flag loads of the other rows.  Call it again
- * (with every plan that sweeps the field) after changing the field's contents. */
+ * It also records, in the plan, which interior rows (y, z) hold a non-zero flag and, per interior
+ * cell, the directions whose walls bounce (4 bytes a cell); the plan's sweeps given this same `flags`
+ * pointer use them instead of the flags.  Call it again (with every plan that sweeps the field) after
+ * changing the field's contents.  While `stream` is being captured, or without the memory, they are
+ * left out and the sweeps take the walls from the flags. */
 int lbm_flags_finalize(const LbmPlan* plan, uint8_t* flags, void* stream);
 
 /* ---- Learned eddy-viscosity closure ----

@@ -338,7 +338,10 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs& a, int x, int y, int
 // near-wall path): the D3Q27 cumulant AA odd sweep went from 80 to 92 registers (3 to 2 blocks)
 // when the per-link boundary data arrived, and the D3Q19 TRT AA odd sweep took 88 (2 blocks, 0.72
 // of the copy bandwidth; 0.92 at 64).  These hot variants are held to register counts checked
-// for spills with -Xptxas -v: 80 (3 blocks), 64 (4) and 48 (5).
+// for spills with -Xptxas -v: 128 (2 blocks), 80 (3), 64 (4) and 48 (5).  The cumulant's three take 64
+// without spilling (odd: 80 before the FP32 copies of the physics and uniform addresses; pull: 90, 192 us
+// for 256x128x128, 155 us at 64).  D3Q27 SRT/TRT AA takes 80 in both parities: at 64 both spill (AA channel
+// 256x128x128 213 us a sweep, 184 us with the odd one at 80, 173 us with both).
 template <class S, int Q, int MK, int PAT> struct SweepMinBlocks { static constexpr int value = 1; };
 template <> struct SweepMinBlocks<float, 27, MK_CUM1, PAT_AA_ODD> { static constexpr int value = 4; };
 template <> struct SweepMinBlocks<double, 19, MK_POP, PAT_PULL> { static constexpr int value = 2; };
@@ -347,8 +350,8 @@ template <> struct SweepMinBlocks<float, 27, MK_CUM1, PAT_AA_EVEN> { static cons
 template <> struct SweepMinBlocks<float, 19, MK_POP, PAT_PULL> { static constexpr int value = 5; };
 template <> struct SweepMinBlocks<float, 19, MK_POP, PAT_AA_ODD> { static constexpr int value = 4; };
 template <> struct SweepMinBlocks<float, 19, MK_POP, PAT_AA_EVEN> { static constexpr int value = 4; };
-template <> struct SweepMinBlocks<float, 27, MK_POP, PAT_AA_ODD> { static constexpr int value = 4; };
-template <> struct SweepMinBlocks<float, 27, MK_POP, PAT_AA_EVEN> { static constexpr int value = 4; };
+template <> struct SweepMinBlocks<float, 27, MK_POP, PAT_AA_ODD> { static constexpr int value = 3; };
+template <> struct SweepMinBlocks<float, 27, MK_POP, PAT_AA_EVEN> { static constexpr int value = 3; };
 template <> struct SweepMinBlocks<float, 19, MK_MRT, PAT_PULL> { static constexpr int value = 4; };
 template <> struct SweepMinBlocks<float, 27, MK_MRT, PAT_PULL> { static constexpr int value = 3; };
 
