@@ -130,8 +130,11 @@ __device__ __forceinline__ void store_row(float* r, const float2 (&v)[MLP_H / 2]
 // FP32 pairs against parameters that one 16-byte shared load brings to the whole warp, and each thread
 // keeps a 4 x 4 tile of the second layer's gradient, so that a sample costs it two 16-byte loads for 16
 // products.  (One gradient entry at a time, with two shared loads per product and the activations in
-// shared memory, took 72 us for 65536 samples.)  Chunks of 64 samples leave 5 blocks per SM.
-__global__ void __launch_bounds__(CHUNK, 5) k_mlp_grad_partial(const float* __restrict__ params,
+// shared memory, took 72 us for 65536 samples.)  Chunks of 64 samples and 4 blocks per SM (as many as the
+// default trainer launches).  Every second chunk the tiles are added to totals of their own, so that a
+// chain of FP32 additions is 128 samples, or the number of such groups, long: one tile over all samples of a
+// block loses digits as they grow in number (3e-3 relative at 2^19 samples a block, 5e-5 so).
+__global__ void __launch_bounds__(CHUNK, 4) k_mlp_grad_partial(const float* __restrict__ params,
                                                            const float* __restrict__ feats,
                                                            const float* __restrict__ target,
                                                            const float* __restrict__ weight, long long n,
@@ -146,12 +149,28 @@ __global__ void __launch_bounds__(CHUNK, 5) k_mlp_grad_partial(const float* __re
     // its bias, column `lane`; second warp: output weights and the other biases, column `lane`
     const int jt = tid >> 3, kt = tid & 7;
     float g2[4][4], g1[MLP_IN + 1];
+    float sum2[4][4], sum1[MLP_IN + 1];
 #pragma unroll
     for (int a = 0; a < 4; ++a)
 #pragma unroll
-        for (int b = 0; b < 4; ++b) g2[a][b] = 0.f;
+        for (int b = 0; b < 4; ++b) g2[a][b] = sum2[a][b] = 0.f;
 #pragma unroll
-    for (int a = 0; a <= MLP_IN; ++a) g1[a] = 0.f;
+    for (int a = 0; a <= MLP_IN; ++a) g1[a] = sum1[a] = 0.f;
+    auto close_group = [&] {
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+#pragma unroll
+            for (int b = 0; b < 4; ++b) {
+                sum2[a][b] += g2[a][b];
+                g2[a][b] = 0.f;
+            }
+#pragma unroll
+        for (int a = 0; a <= MLP_IN; ++a) {
+            sum1[a] += g1[a];
+            g1[a] = 0.f;
+        }
+    };
+    bool second = false;
     double loss = 0.0;
     const float scale = params[MLP_SCALE];
     __syncthreads();
@@ -244,20 +263,23 @@ __global__ void __launch_bounds__(CHUNK, 5) k_mlp_grad_partial(const float* __re
             }
         }
         __syncthreads();
+        if (second) close_group();
+        second = !second;
     }
+    close_group();
     float* out = partial + (long long)blockIdx.x * MLP_TRAINED;
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int k = 0; k < 4; ++k) out[MLP_W2 + (4 * jt + i) * MLP_H + 4 * kt + k] = g2[i][k];
+        for (int k = 0; k < 4; ++k) out[MLP_W2 + (4 * jt + i) * MLP_H + 4 * kt + k] = sum2[i][k];
     if (tid < 32) {
 #pragma unroll
-        for (int i = 0; i < MLP_IN; ++i) out[MLP_W1 + i * MLP_H + lane] = g1[i];
-        out[MLP_B1 + lane] = g1[MLP_IN];
+        for (int i = 0; i < MLP_IN; ++i) out[MLP_W1 + i * MLP_H + lane] = sum1[i];
+        out[MLP_B1 + lane] = sum1[MLP_IN];
     } else {
-        out[MLP_W3 + lane] = g1[0];
-        out[MLP_B2 + lane] = g1[1];
-        if (lane == 0) out[MLP_B3] = g1[2];
+        out[MLP_W3 + lane] = sum1[0];
+        out[MLP_B2 + lane] = sum1[1];
+        if (lane == 0) out[MLP_B3] = sum1[2];
     }
     // block loss: fixed-order tree in shared memory
     __shared__ double red[CHUNK];
