@@ -133,7 +133,10 @@ class MLPClosure:
     def _workspace(self):
         """The reduction workspace of loss_and_grad, kept with the closure: allocating and freeing one
         per call waits for the device twice.  One per device, stream and thread, so that calls that may
-        overlap do not share it; the least recently used is given back when there are more than a few."""
+        overlap do not share it; the least recently used is given back when there are more than a few,
+        which a captured graph would not survive: capture takes a workspace of the caller's own."""
+        if torch.cuda.is_current_stream_capturing():
+            raise N.LbmError("loss_and_grad needs a trainer of the caller's own while a graph is captured")
         key = (torch.cuda.current_device(), torch.cuda.current_stream().cuda_stream, threading.get_ident())
         with self._workspace_lock:
             w = self._workspaces.pop(key, None) or _Trainer()

@@ -50,3 +50,28 @@ def test_streams_and_threads_do_not_share_it(cuda):
         t.join()
     assert all(torch.equal(a, b) for a, b in zip(got, want))
     assert len(clo._workspaces) <= clo._MAX_WORKSPACES
+
+
+def test_a_captured_graph_does_not_hold_the_kept_workspace(cuda):
+    """The kept workspace may be given back while a graph that was captured with it lives on, so capture
+    without a workspace of the caller's own is refused, also on a stream the call was warmed on."""
+    clo = C.MLPClosure(seed=3)
+    feats, target, _ = _samples(1000, 9)
+    stream, own = torch.cuda.Stream(), C._Trainer()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream):
+        want = clo.loss_and_grad(feats, target)[1]
+        clo.loss_and_grad(feats, target, trainer=own)
+    torch.cuda.synchronize()
+    refused, graph = False, torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        try:
+            clo.loss_and_grad(feats, target)
+        except RuntimeError:
+            refused = True
+        grad = clo.loss_and_grad(feats, target, trainer=own)[1]
+    assert refused
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(grad, want)
+    assert torch.equal(clo.loss_and_grad(feats, target)[1], want)
