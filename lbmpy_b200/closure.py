@@ -226,6 +226,6 @@ class _Trainer:
 
     def __del__(self):
         h = getattr(self, "handle", None)
-        if h is not None and h.value and N._lib is not None:
+        if h is not None and h.value and N is not None and N._lib is not None:
             N._lib.lbm_mlp_destroy(h)
             self.handle = None

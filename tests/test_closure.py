@@ -115,3 +115,13 @@ def test_host_closure_collision_matches_oracle(host, force, galilean):  # noqa: 
         assert np.abs(h - ref).max() / scale < 2e-7
         oms.append(om)
     assert min(oms) < 1.99 - 1e-3            # the closure is active: omega below the base rate
+
+
+def test_a_workspace_left_at_interpreter_exit_is_quiet(monkeypatch):
+    """At exit the module's globals may be gone before the workspaces that closures keep."""
+    import ctypes
+    from lbmpy_b200 import closure as C
+    w = C._Trainer.__new__(C._Trainer)
+    w.handle = ctypes.c_void_p(1)
+    monkeypatch.setattr(C, "N", None)
+    w.__del__()
