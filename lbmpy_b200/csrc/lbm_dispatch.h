@@ -5,6 +5,7 @@
 #include <atomic>
 #include <type_traits>
 
+#include "lbm_launch.h"
 #include "lbm_quad.cuh"
 #include "lbm_staged.cuh"
 
@@ -12,23 +13,6 @@ namespace lbm {
 
 using SweepLauncher = cudaError_t (*)(const SweepArgs&, dim3, dim3, cudaStream_t);
 using MacroLauncher = cudaError_t (*)(const MacroArgs&, dim3, dim3, cudaStream_t);
-
-// Launches a kernel that begins with chain_wait(): it may start while the kernel before it in the stream
-// still runs, and waits for it there.
-template <class... KA, class... A>
-cudaError_t launch_chained(void (*kernel)(KA...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, const A&... args) {
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t c = {};
-    c.gridDim = grid;
-    c.blockDim = block;
-    c.dynamicSmemBytes = smem;
-    c.stream = s;
-    c.attrs = &attr;
-    c.numAttrs = 1;
-    return cudaLaunchKernelEx(&c, kernel, KA(args)...);
-}
 
 template <class S, class R, int Q, int MK, int PAT>
 cudaError_t launch_sweep(const SweepArgs& a, dim3 grid, dim3 block, cudaStream_t s) {
