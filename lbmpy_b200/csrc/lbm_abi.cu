@@ -506,30 +506,11 @@ __global__ void k_flags_finalize(Grid g) {
 // Wall words of a finalized flag field (WALL_* in lbm_common.cuh), one per interior cell.
 template <int Q>
 __global__ void __launch_bounds__(256) k_wall_words(Grid g, uint32_t* words) {
-    using L = Lat<Q>;
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     const int y = blockIdx.y * blockDim.y + threadIdx.y;
     const int z = blockIdx.z;
     if (x >= g.nx || y >= g.ny) return;
-    const uint8_t* cell = g.flags + ((x + 1) + (y + 1) * g.fsy + (z + 1) * g.fsz);
-    const int fl = *cell;
-    uint32_t w = 0;
-    if (fl & FLAG_TYPE_MASK) {
-        w = WALL_SELF;
-    } else if (fl & FLAG_NEAR_WALL) {
-        const NbrOffsets fo = flag_offsets(g, x, y, z);
-        unsigned types = 0;   // bit t: a link to a cell of type t
-#pragma unroll
-        for (int i = 1; i < Q; ++i) {
-            const int t = cell[fo.off(-L::cx(i), -L::cy(i), -L::cz(i))] & FLAG_TYPE_MASK;
-            types |= 1u << t;
-            if (t == FLAG_NOSLIP || flag_is_ubb(t)) w |= 1u << i;
-        }
-        if (types & ((1u << FLAG_FIXED_DENSITY) | (1u << FLAG_FIXED_DENSITY1))) w |= WALL_FIXED_DENSITY;
-        if (types >> FLAG_FREE_SLIP) w |= WALL_PER_LINK;
-        if ((types >> FLAG_UBB0) & ((1u << MAX_UBB) - 1u)) w |= WALL_UBB;
-    }
-    words[size_t(x) + size_t(g.nx) * (size_t(y) + size_t(g.ny) * z)] = w;
+    words[size_t(x) + size_t(g.nx) * (size_t(y) + size_t(g.ny) * z)] = wall_word_of_flags<Q>(g, x, y, z);
 }
 
 cudaError_t launch_wall_words(int q, const Grid& g, uint32_t* words, cudaStream_t s) {

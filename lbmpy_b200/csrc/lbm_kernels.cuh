@@ -15,6 +15,7 @@
 // would have copied (the f_out location of advanced_streaming/indexing.py:12-183).
 #pragma once
 #include "lbm_collide.cuh"
+#include "lbm_walls.cuh"
 
 namespace lbm {
 
@@ -435,15 +436,6 @@ __global__ void __launch_bounds__(256) k_ubb_density(const SweepArgs a, R* rho_o
     const int z = blockIdx.z;
     if (x >= g.nx || y >= g.ny) return;
     if (!(wall_word<Q>(g, x, y, z) & WALL_UBB)) return;
-    if (g.walls == nullptr) {
-        const NbrOffsets fo = flag_offsets(g, x, y, z);
-        const uint8_t* fl = g.flags + ((x + 1) + (y + 1) * g.fsy + (z + 1) * g.fsz);
-        bool moving = false;
-#pragma unroll
-        for (int i = 1; i < Q; ++i)
-            if (flag_is_ubb(fl[fo.off(-L::cx(i), -L::cy(i), -L::cz(i))] & FLAG_TYPE_MASK)) moving = true;
-        if (!moving) return;
-    }
     NbrOffsets nb;
     nb.init(g, x, y, z);
     const int cell = (x + 1) + (y + 1) * g.sy + (z + 1) * g.sz;
