@@ -206,12 +206,36 @@ int lbm_plan_set_links(LbmPlan* plan, const LbmLinkTables* tables);
 /* Sets bit 7 on every fluid cell of `flags` (device, layout above) that has a boundary
  * neighbour along the plan's stencil, honouring periodicity.  Replaces the link-list setup of
  * LatticeBoltzmannBoundaryHandling (boundaries/boundaryhandling.py:15-155).
- * It also records, in the plan, which interior rows (y, z) hold a non-zero flag and, per interior
- * cell, the directions whose walls bounce (4 bytes a cell); the plan's sweeps given this same `flags`
- * pointer use them instead of the flags.  Call it again (with every plan that sweeps the field) after
- * changing the field's contents.  While `stream` is being captured, or without the memory, they are
- * left out and the sweeps take the walls from the flags. */
+ * It also records, in the plan, which interior rows (y, z) hold a non-zero flag; the plan's
+ * sweeps given this same `flags` pointer skip the flag loads of the other rows.  Call it again
+ * (with every plan that sweeps the field) after changing the field's contents. */
 int lbm_flags_finalize(const LbmPlan* plan, uint8_t* flags, void* stream);
+
+/* The walls of one finalized flag field in the form the sweeps read fastest: a bit per interior row that
+ * holds a non-zero flag, and per interior cell a word with the directions whose walls bounce.  All device
+ * memory is the caller's: lbm_walls_size gives the length (32-bit words) of the buffer that lbm_walls_build
+ * fills from `flags`, which must be finalized for the plan's stencil and periodicity.  The result describes
+ * the flags as they are then; build it again, into the same or another buffer, after changing them.  It belongs to
+ * the flag field and not to the plan: every plan of the same stencil, dims and periodicity may sweep with
+ * it, and fields with different walls may share a plan.  lbm_walls_slab describes the interior planes [z0, z0 + nz) of a
+ * domain that is not periodic in z, on the same memory.
+ * No lbmpy counterpart (its boundary kernels walk link lists, boundaries/boundaryhandling.py:15-155). */
+typedef struct LbmWalls {
+    const uint8_t* flags;
+    const uint32_t* rows;
+    const uint32_t* words;
+    int32_t stencil;
+    int32_t dims[3];
+    int32_t periodic[3];
+} LbmWalls;
+int lbm_walls_size(const LbmPlan* plan, int64_t* words);
+int lbm_walls_build(const LbmPlan* plan, const uint8_t* flags, uint32_t* buffer, LbmWalls* out, void* stream);
+int lbm_walls_slab(const LbmWalls* whole, int z0, int nz, LbmWalls* out);
+/* lbm_sweep and lbm_run with walls->flags as the flags; the result is the same. */
+int lbm_sweep_walls(const LbmPlan* plan, const void* src, void* dst, const int64_t strides[4], const LbmWalls* walls,
+                    int parity, float* omega_out, void* stream);
+int lbm_run_walls(const LbmPlan* plan, void* a, void* b, const int64_t strides[4], const LbmWalls* walls,
+                  int first_parity, int steps, int* result_in_b, void* stream);
 
 /* ---- Learned eddy-viscosity closure ----
  * sgs = LBM_SGS_MLP replaces the closed-form eddy viscosity of lbmpy's Smagorinsky model

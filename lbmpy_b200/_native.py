@@ -26,7 +26,8 @@ MLP_PARAMS = 1442
 EXPORTS = ("lbm_plan_create", "lbm_plan_destroy", "lbm_plan_update", "lbm_plan_status", "lbm_sweep_variant",
            "lbm_sweep", "lbm_run",
            "lbm_set_equilibrium", "lbm_get_macroscopic", "lbm_reduce_conserved", "lbm_reduce_conserved_noalloc",
-           "lbm_flags_finalize", "lbm_plan_set_links", "lbm_closure_set_weights", "lbm_closure_features", "lbm_mlp_forward",
+           "lbm_flags_finalize", "lbm_walls_size", "lbm_walls_build", "lbm_walls_slab", "lbm_sweep_walls", "lbm_run_walls",
+           "lbm_plan_set_links", "lbm_closure_set_weights", "lbm_closure_features", "lbm_mlp_forward",
            "lbm_mlp_create", "lbm_mlp_destroy", "lbm_mlp_loss_grad", "lbm_mlp_adam", "lbm_batch_create", "lbm_batch_sweep", "lbm_batch_info", "lbm_batch_destroy",
            "lbm_sparse_sweep", "lbm_sparse_set_equilibrium", "lbm_sparse_get_macroscopic", "lbm_sparse_ubb",
            "lbm_plan_set_stage_wait", "lbm_halo_copy",
@@ -60,6 +61,11 @@ class LbmPlanDesc(ctypes.Structure):
 class LbmLinkTables(ctypes.Structure):
     _fields_ = [("cell_block", ctypes.c_void_p), ("n_blocks", ctypes.c_int64), ("ubb_velocity", ctypes.c_void_p),
                 ("ubb_mask", ctypes.c_uint32), ("link_code", ctypes.c_void_p), ("link_value", ctypes.c_void_p)]
+
+
+class LbmWalls(ctypes.Structure):
+    _fields_ = [("flags", ctypes.c_void_p), ("rows", ctypes.c_void_p), ("words", ctypes.c_void_p),
+                ("stencil", ctypes.c_int32), ("dims", ctypes.c_int32 * 3), ("periodic", ctypes.c_int32 * 3)]
 
 
 class LbmDomainDesc(ctypes.Structure):
@@ -112,6 +118,12 @@ def lib():
         L.lbm_reduce_conserved_noalloc.argtypes = [ctypes.POINTER(LbmPlanDesc), vp, i64p, vp, ctypes.c_int,
                                                    ctypes.POINTER(ctypes.c_double), vp]
         L.lbm_flags_finalize.argtypes = [vp, vp, vp]
+        wp = ctypes.POINTER(LbmWalls)
+        L.lbm_walls_size.argtypes = [vp, i64p]
+        L.lbm_walls_build.argtypes = [vp, vp, vp, wp, vp]
+        L.lbm_walls_slab.argtypes = [wp, ctypes.c_int, ctypes.c_int, wp]
+        L.lbm_sweep_walls.argtypes = [vp, vp, vp, i64p, wp, ctypes.c_int, vp, vp]
+        L.lbm_run_walls.argtypes = [vp, vp, vp, i64p, wp, ctypes.c_int, ctypes.c_int, ctypes.POINTER(ctypes.c_int), vp]
         L.lbm_plan_set_links.argtypes = [vp, ctypes.POINTER(LbmLinkTables)]
         L.lbm_closure_set_weights.argtypes = [vp, ctypes.c_int, vp]
         L.lbm_closure_features.argtypes = [vp, ctypes.c_int64, vp, vp]
@@ -162,6 +174,20 @@ def check(rc: int, what: str = ""):
 
 def i64_array(values):
     return (ctypes.c_int64 * len(values))(*[int(v) for v in values])
+
+
+class Walls:
+    """An LbmWalls and the tensors whose device memory it points to."""
+
+    def __init__(self, native: LbmWalls, tensors):
+        self.native = native
+        self.tensors = tuple(tensors)
+
+    def slab(self, z0: int, nz: int) -> "Walls":
+        """The walls of interior planes [z0, z0 + nz)."""
+        out = LbmWalls()
+        check(lib().lbm_walls_slab(ctypes.byref(self.native), int(z0), int(nz), ctypes.byref(out)), "lbm_walls_slab")
+        return Walls(out, self.tensors)
 
 
 class Plan:

@@ -273,6 +273,7 @@ class LatticeBoltzmannBoundaryHandling:
         self._fixed_densities: List[float] = []
         self._dev: Optional[torch.Tensor] = None
         self._finalized_for = None
+        self._walls: Optional[N.Walls] = None
         self._links = None          # device link tables (LbmLinkTables and the tensors they point to)
         self._link_objs: List = []  # FreeSlip / outflow / Bouzidi objects, indexed by self._obj
         self._obj = np.full((ez, ey, ex), -1, dtype=np.int16)
@@ -612,12 +613,34 @@ class LatticeBoltzmannBoundaryHandling:
         key = (int(plan.desc.stencil), tuple(plan.desc.periodic))
         if self._dev is None or self._finalized_for != key:
             t = torch.from_numpy(self._host.copy()).to(self.device).permute(2, 1, 0)
-            N.check(N.lib().lbm_flags_finalize(plan.handle, ctypes.c_void_p(t.data_ptr()),
-                                               ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)),
+            stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+            N.check(N.lib().lbm_flags_finalize(plan.handle, ctypes.c_void_p(t.data_ptr()), stream),
                     "lbm_flags_finalize")
+            self._walls = self._build_walls(plan, t, stream)
             self._dev = t
             self._finalized_for = key
         return self._dev
+
+    @staticmethod
+    def _build_walls(plan, flags, stream) -> Optional[N.Walls]:
+        """The walls of a finalized flag field, in memory of torch's allocator (4 bytes a cell; cudaMalloc on
+        the first sweep of a new domain took longer than the sweep).  None without the memory: the sweeps
+        then take the walls from the flags."""
+        n = ctypes.c_int64(0)
+        N.check(N.lib().lbm_walls_size(plan.handle, ctypes.byref(n)), "lbm_walls_size")
+        try:
+            buffer = torch.empty(n.value, dtype=torch.int32, device=flags.device)
+        except torch.cuda.OutOfMemoryError:
+            return None
+        w = N.LbmWalls()
+        N.check(N.lib().lbm_walls_build(plan.handle, ctypes.c_void_p(flags.data_ptr()),
+                                        ctypes.c_void_p(buffer.data_ptr()), ctypes.byref(w), stream), "lbm_walls_build")
+        return N.Walls(w, (flags, buffer))
+
+    @property
+    def walls(self) -> Optional[N.Walls]:
+        """The walls of the field that flags() returned last, for the sweeps (LbKernel.bind)."""
+        return self._walls
 
     def __call__(self, *args, **kwargs):
         """Boundaries are applied inside the sweep; calling the handling is a no-op kept for

@@ -34,9 +34,8 @@ struct LbmPlan {
     int block_x;           // x extent of the one-cell sweep's 256-thread blocks, 0 automatic (LBM_B200_BX)
     int sms;               // multiprocessors of the plan's device
     unsigned* status;      // device status word (lbm_plan_status), inside the reduction scratch
-    mutable uint32_t* rowmask;             // row summary of the flag field last finalized with this plan
+    uint32_t* rowmask;     // row summary of the flag field last finalized with this plan
     mutable const uint8_t* rowmask_flags;  // that flag field (sweeps given it use the summary)
-    mutable uint32_t* walls;               // its wall words, behind the row summary
     void* ubb_rho;         // compressible + moving UBB walls: density gathered before the sweep
     const int* ubb_block;  // per-link boundary tables (lbm_plan_set_links), caller-owned
     const double* ubb_link_vel;
@@ -209,9 +208,9 @@ SweepLauncher pair_launcher(const LbmPlan* p, int pat) {
 
 size_t store_size(int store) { return store == ST_F64 ? 8 : (store == ST_F32 ? 4 : 2); }
 
-size_t rowmask_bytes(const LbmPlan* p) {
-    return sizeof(uint32_t) * ((size_t(p->desc.dims[1]) * p->desc.dims[2] + 31) / 32);
-}
+// Words of a row summary: a bit per row, every plane starting a new word (a slab of planes has its part).
+size_t row_words(const int32_t dims[3]) { return (size_t(dims[1]) + 31) / 32 * size_t(dims[2]); }
+size_t rowmask_bytes(const LbmPlan* p) { return sizeof(uint32_t) * row_words(p->desc.dims); }
 
 SweepLauncher quad_launcher(const LbmPlan* p, int pat) {
     if (p->q == 19 && p->mk == MK_POP) return sweep_quad_q19_pop(p->store, pat);
@@ -464,7 +463,7 @@ int ensure_ubb_buffer(LbmPlan* p) {
     return LBM_OK;
 }
 
-// Row summary of a finalized flag field: bit y + ny*z for every interior row with a non-zero flag.
+// Row summary of a finalized flag field (Grid::rowmask): a bit for every interior row with a non-zero flag.
 __global__ void k_row_mask(Grid g, uint32_t* mask) {
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= g.ny * g.nz) return;
@@ -472,7 +471,7 @@ __global__ void k_row_mask(Grid g, uint32_t* mask) {
     const uint8_t* row = g.flags + 1 + (y + 1) * g.fsy + (z + 1) * g.fsz;
     for (int x = 0; x < g.nx; ++x)
         if (row[x] != 0) {
-            atomicOr(mask + (r >> 5), 1u << (r & 31));
+            atomicOr(mask + (y >> 5) + ((g.ny + 31) >> 5) * z, 1u << (y & 31));
             break;
         }
 }
@@ -511,6 +510,14 @@ __global__ void __launch_bounds__(256) k_wall_words(Grid g, uint32_t* words) {
     const int z = blockIdx.z;
     if (x >= g.nx || y >= g.ny) return;
     words[size_t(x) + size_t(g.nx) * (size_t(y) + size_t(g.ny) * z)] = wall_word_of_flags<Q>(g, x, y, z);
+}
+
+cudaError_t launch_row_mask(const Grid& g, uint32_t* rows, cudaStream_t s) {
+    const int32_t dims[3] = {g.nx, g.ny, g.nz};
+    const cudaError_t e = cudaMemsetAsync(rows, 0, sizeof(uint32_t) * row_words(dims), s);
+    if (e != cudaSuccess) return e;
+    k_row_mask<<<(g.ny * g.nz + 255) / 256, 256, 0, s>>>(g, rows);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_wall_words(int q, const Grid& g, uint32_t* words, cudaStream_t s) {
@@ -759,7 +766,6 @@ int lbm_plan_create(const LbmPlanDesc* desc, LbmPlan** out) {
     p->ubb_rho = nullptr;
     p->rowmask = nullptr;
     p->rowmask_flags = nullptr;
-    p->walls = nullptr;
     if (sweep_launcher(p, PAT_PULL) == nullptr) {
         cudaFree(p->partial);
         delete p;
@@ -769,6 +775,13 @@ int lbm_plan_create(const LbmPlanDesc* desc, LbmPlan** out) {
         cudaFree(p->partial);
         delete p;
         return rc2;
+    }
+    e = cudaMalloc(&p->rowmask, rowmask_bytes(p));
+    if (e != cudaSuccess) {
+        cudaFree(p->partial);
+        if (p->ubb_rho) cudaFree(p->ubb_rho);
+        delete p;
+        return cuda_fail(e, "cudaMalloc(row summary)");
     }
     *out = p;
     return LBM_OK;
@@ -782,6 +795,8 @@ int lbm_plan_update(LbmPlan* p, const LbmPlanDesc* desc) {
         return fail(LBM_E_INVALID, "lbm_plan_update may only change physical parameters");
     int rc = validate_desc(desc);
     if (rc) return rc;
+    // a row summary of near-wall cells under another wrap no longer fits
+    if (memcmp(desc->periodic, p->desc.periodic, sizeof(desc->periodic)) != 0) p->rowmask_flags = nullptr;
     p->desc = *desc;
     p->mk = method_kind(desc);
     fill_physics(p, desc);
@@ -830,7 +845,8 @@ static int sweep_variant(const LbmPlan* p, const void* src, const void* dst, con
 
 // Launch without re-validating (arguments checked by the caller).
 static int launch_sweep_checked(const LbmPlan* p, const void* src, void* dst, const int64_t strides[4],
-                                const uint8_t* flags, int parity, float* omega_out, cudaStream_t stream) {
+                                const uint8_t* flags, const LbmWalls* walls, int parity, float* omega_out,
+                                cudaStream_t stream) {
     const int pat = pattern_kind(p, parity);
     SweepArgs a;
     a.g = make_grid(p, strides, flags);
@@ -847,12 +863,11 @@ static int launch_sweep_checked(const LbmPlan* p, const void* src, void* dst, co
     a.ubb_link_vel = p->ubb_link_vel;
     a.link_code = p->link_code;
     a.link_value = p->link_value;
-    if (flags != nullptr && flags == p->rowmask_flags) {
-        // Not periodic in x, a domain has boundary cells at the ends of every row: the summary would only
-        // delay the wall words, which the sweeps then ask for with the populations (as batches do).
-        a.g.rowmask = p->desc.periodic[0] ? p->rowmask : nullptr;
-        a.g.walls = p->walls;
-    }
+    // Not periodic in x, a domain has boundary cells at the ends of every row: the summary would only
+    // delay the wall words, which the sweeps then ask for with the populations (as batches do).
+    if (p->desc.periodic[0])
+        a.g.rowmask = walls != nullptr ? walls->rows : flags != nullptr && flags == p->rowmask_flags ? p->rowmask : nullptr;
+    if (walls != nullptr) a.g.walls = walls->words;
     if (flags != nullptr && p->ubb_rho != nullptr && needs_ubb_density(&p->desc, p->ubb_link_mask)) {
         UbbLauncher U = p->q == 19 ? ubb_launcher_q<19>(p->store, pat) : ubb_launcher_q<27>(p->store, pat);
         if (U == nullptr) return fail(LBM_E_UNSUPPORTED, "no wall-density kernel for this storage type / pattern");
@@ -912,7 +927,28 @@ int lbm_sweep(const LbmPlan* p, const void* src, void* dst, const int64_t stride
     int rc = validate_sweep(p, src, dst, strides, flags, omega_out);
     if (rc) return rc;
     if (parity != 0 && parity != 1) return fail(LBM_E_INVALID, "parity must be 0 (EVEN) or 1 (ODD)");
-    return launch_sweep_checked(p, src, dst, strides, flags, parity, omega_out, static_cast<cudaStream_t>(stream));
+    return launch_sweep_checked(p, src, dst, strides, flags, nullptr, parity, omega_out,
+                                static_cast<cudaStream_t>(stream));
+}
+
+static int check_walls(const LbmPlan* p, const LbmWalls* w) {
+    if (p == nullptr) return fail(LBM_E_INVALID, "plan is NULL");
+    if (w == nullptr || w->flags == nullptr || w->rows == nullptr || w->words == nullptr)
+        return fail(LBM_E_INVALID, "walls must be filled by lbm_walls_build or lbm_walls_slab");
+    if (w->stencil != p->desc.stencil || memcmp(w->dims, p->desc.dims, sizeof(w->dims)) != 0 ||
+        memcmp(w->periodic, p->desc.periodic, sizeof(w->periodic)) != 0)
+        return fail(LBM_E_INVALID, "the walls were built for another stencil, domain or periodicity");
+    return LBM_OK;
+}
+
+int lbm_sweep_walls(const LbmPlan* p, const void* src, void* dst, const int64_t strides[4], const LbmWalls* walls,
+                    int parity, float* omega_out, void* stream) {
+    int rc = check_walls(p, walls);
+    if (rc) return rc;
+    if ((rc = validate_sweep(p, src, dst, strides, walls->flags, omega_out))) return rc;
+    if (parity != 0 && parity != 1) return fail(LBM_E_INVALID, "parity must be 0 (EVEN) or 1 (ODD)");
+    return launch_sweep_checked(p, src, dst, strides, walls->flags, walls, parity, omega_out,
+                                static_cast<cudaStream_t>(stream));
 }
 
 int lbm_sweep_variant(const LbmPlan* p, const void* src, const void* dst, const int64_t strides[4], int parity,
@@ -940,8 +976,8 @@ int lbm_plan_status(LbmPlan* p, uint32_t* status, int clear) {
     return LBM_OK;
 }
 
-int lbm_run(const LbmPlan* p, void* a, void* b, const int64_t strides[4], const uint8_t* flags, int first_parity,
-            int steps, int* result_in_b, void* stream) {
+static int run_steps(const LbmPlan* p, void* a, void* b, const int64_t strides[4], const uint8_t* flags,
+                     const LbmWalls* walls, int first_parity, int steps, int* result_in_b, void* stream) {
     if (p == nullptr) return fail(LBM_E_INVALID, "plan is NULL");
     if (steps < 0) return fail(LBM_E_INVALID, "steps must be >= 0");
     if (first_parity != 0 && first_parity != 1) return fail(LBM_E_INVALID, "parity must be 0 (EVEN) or 1 (ODD)");
@@ -953,13 +989,24 @@ int lbm_run(const LbmPlan* p, void* a, void* b, const int64_t strides[4], const 
     int parity = first_parity;
     int in_b = 0;
     for (int t = 0; t < steps; ++t) {
-        rc = launch_sweep_checked(p, src, dst, strides, flags, parity, nullptr, static_cast<cudaStream_t>(stream));
+        rc = launch_sweep_checked(p, src, dst, strides, flags, walls, parity, nullptr, static_cast<cudaStream_t>(stream));
         if (rc) return rc;
         if (inplace) parity ^= 1;
         else { void* tmp = src; src = dst; dst = tmp; in_b ^= 1; }
     }
     if (result_in_b) *result_in_b = in_b;
     return LBM_OK;
+}
+
+int lbm_run(const LbmPlan* p, void* a, void* b, const int64_t strides[4], const uint8_t* flags, int first_parity,
+            int steps, int* result_in_b, void* stream) {
+    return run_steps(p, a, b, strides, flags, nullptr, first_parity, steps, result_in_b, stream);
+}
+
+int lbm_run_walls(const LbmPlan* p, void* a, void* b, const int64_t strides[4], const LbmWalls* walls,
+                  int first_parity, int steps, int* result_in_b, void* stream) {
+    int rc = check_walls(p, walls);
+    return rc ? rc : run_steps(p, a, b, strides, walls->flags, walls, first_parity, steps, result_in_b, stream);
 }
 
 static int macro_common(const LbmPlan* p, const void* pdfs, const int64_t strides[4], const void* rho,
@@ -1072,29 +1119,54 @@ int lbm_flags_finalize(const LbmPlan* p, uint8_t* flags, void* stream) {
     else k_flags_finalize<27><<<grid, block, 0, st>>>(g);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(e, "flag finalize launch");
-    // The row summary and the wall words the sweeps of this plan use with this flag field.  Without the
-    // memory for them (or while a graph is being captured, when it cannot be allocated) the sweeps
-    // take the walls from the flags.
+    // the row summary the sweeps of this plan use with this flag field
     p->rowmask_flags = nullptr;
-    const size_t rows = rowmask_bytes(p), cells = size_t(g.nx) * g.ny * g.nz;
-    if (p->rowmask == nullptr) {
-        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-        if (cudaStreamIsCapturing(st, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone ||
-            cudaMalloc(&p->rowmask, rows + sizeof(uint32_t) * cells) != cudaSuccess) {
-            p->rowmask = nullptr;
-            cudaGetLastError();
-            return LBM_OK;
-        }
-        p->walls = p->rowmask + rows / sizeof(uint32_t);
-    }
-    e = cudaMemsetAsync(p->rowmask, 0, rows, st);
-    if (e != cudaSuccess) return cuda_fail(e, "clearing the row summary");
-    k_row_mask<<<(g.ny * g.nz + 255) / 256, 256, 0, st>>>(g, p->rowmask);
-    e = cudaGetLastError();
+    e = launch_row_mask(g, p->rowmask, st);
     if (e != cudaSuccess) return cuda_fail(e, "row summary launch");
-    e = launch_wall_words(p->q, g, p->walls, st);
-    if (e != cudaSuccess) return cuda_fail(e, "wall word launch");
     p->rowmask_flags = flags;
+    return LBM_OK;
+}
+
+int lbm_walls_size(const LbmPlan* p, int64_t* words) {
+    if (p == nullptr || words == nullptr) return fail(LBM_E_INVALID, "plan and words must not be NULL");
+    const int32_t* n = p->desc.dims;
+    *words = int64_t(row_words(n)) + int64_t(n[0]) * n[1] * n[2];
+    return LBM_OK;
+}
+
+int lbm_walls_build(const LbmPlan* p, const uint8_t* flags, uint32_t* buffer, LbmWalls* out, void* stream) {
+    if (p == nullptr || out == nullptr) return fail(LBM_E_INVALID, "plan and out must not be NULL");
+    int rc;
+    if ((rc = check_device(p))) return rc;
+    if ((rc = check_device_ptr(p, flags, "flags", false))) return rc;
+    if ((rc = check_device_ptr(p, buffer, "buffer", false))) return rc;
+    const int64_t s[4] = {1, p->desc.dims[0] + 2, int64_t(p->desc.dims[0] + 2) * (p->desc.dims[1] + 2), 0};
+    const Grid g = make_grid(p, s, flags);
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    uint32_t* words = buffer + row_words(p->desc.dims);
+    cudaError_t e = launch_row_mask(g, buffer, st);
+    if (e == cudaSuccess) e = launch_wall_words(p->q, g, words, st);
+    if (e != cudaSuccess) return cuda_fail(e, "wall word launch");
+    out->flags = flags;
+    out->rows = buffer;
+    out->words = words;
+    out->stencil = p->desc.stencil;
+    memcpy(out->dims, p->desc.dims, sizeof(out->dims));
+    memcpy(out->periodic, p->desc.periodic, sizeof(out->periodic));
+    return LBM_OK;
+}
+
+int lbm_walls_slab(const LbmWalls* whole, int z0, int nz, LbmWalls* out) {
+    if (whole == nullptr || out == nullptr) return fail(LBM_E_INVALID, "whole and out must not be NULL");
+    if (z0 < 0 || nz < 1 || z0 > whole->dims[2] - nz)
+        return fail(LBM_E_INVALID, "planes [%d, %d) are not inside a domain of %d", z0, z0 + nz, whole->dims[2]);
+    if (whole->periodic[2]) return fail(LBM_E_INVALID, "a slab of a domain periodic in z has other walls at its ends");
+    const int64_t nx = whole->dims[0], ny = whole->dims[1];
+    *out = *whole;
+    out->flags += (nx + 2) * (ny + 2) * z0;
+    out->rows += (ny + 31) / 32 * z0;
+    out->words += nx * ny * z0;
+    out->dims[2] = nz;
     return LBM_OK;
 }
 

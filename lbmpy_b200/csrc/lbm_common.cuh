@@ -229,8 +229,8 @@ struct Grid {
     int periodic;          // bit 0 x, bit 1 y, bit 2 z
     const uint8_t* flags;  // (nx+2)*(ny+2)*(nz+2), x fastest, or nullptr
     int fsy, fsz;          // flag strides
-    // Bit y + ny*z set: interior row (y, z) holds a cell whose flag is non-zero (a boundary cell
-    // or a fluid cell next to one).  nullptr: every row may.  Sweeps skip the flag loads of the
+    // Bit y % 32 of word y / 32 + z * ceil(ny / 32) set: interior row (y, z) holds a cell whose flag is
+    // non-zero (a boundary cell or a fluid cell next to one).  nullptr: every row may.  Sweeps skip the flag loads of the
     // other rows, so that a fluid cell's populations are not held up behind its flag.
     const uint32_t* rowmask;
     // Wall words of the interior cells, x fastest (see WALL_*); nullptr: the sweeps take the walls
@@ -265,8 +265,7 @@ struct SweepArgs {
 // Whether interior row (y, z) may hold a cell with a non-zero flag.
 __device__ __forceinline__ bool row_flagged(const Grid& g, int y, int z) {
     if (g.rowmask == nullptr) return true;
-    const unsigned r = unsigned(y) + unsigned(g.ny) * unsigned(z);
-    return (g.rowmask[r >> 5] >> (r & 31u)) & 1u;
+    return (g.rowmask[(unsigned(y) >> 5) + ((unsigned(g.ny) + 31u) >> 5) * unsigned(z)] >> (unsigned(y) & 31u)) & 1u;
 }
 
 // Neighbour offsets in elements for c in {-1, 0, +1} along each axis, with periodic wrap.

@@ -263,8 +263,9 @@ class DistributedLatticeBoltzmannStep:
         for z0, nz in ((0, 1), (zl - 1, 1), (1, zl - 2)):    # interior planes [z0, z0 + nz)
             view = loc.pdfs[:, :, z0:z0 + nz + 2]
             fl = flags[:, :, z0:z0 + nz + 2] if flags is not None else None
+            walls = bh.walls.slab(z0, nz) if flags is not None and bh.walls is not None else None
             b = k.bind(view, per, fl, bh.ubb_velocities, loc.kernel_params, fixed_density=bh.fixed_density,
-                       ubb_options=bh.ubb_options)
+                       ubb_options=bh.ubb_options, walls=walls)
             parts.append((z0 * view.stride(2) * view.element_size(), b))
         self._split = (whole, parts)
         return parts

@@ -143,19 +143,29 @@ def _stream_handle(stream) -> Optional[int]:
 
 class BoundSweep:
     """A sweep with its plan, strides, flags and stream resolved once: launching it costs one
-    ctypes call (the per-step path of LatticeBoltzmannStep)."""
+    ctypes call (the per-step path of LatticeBoltzmannStep).  With `walls` (the N.Walls of `flags`) the
+    sweeps read the walls from there."""
 
-    def __init__(self, plan: N.Plan, strides, flags, stream_handle):
+    def __init__(self, plan: N.Plan, strides, flags, stream_handle, walls: Optional[N.Walls] = None):
         self.plan = plan
         self._strides = N.i64_array(strides)
-        self._flags = ctypes.c_void_p(flags.data_ptr() if flags is not None else None)
         self._flags_ref = flags
+        self._walls_ref = walls
         self._stream = ctypes.c_void_p(stream_handle)
         self._lib = N.lib()
+        if walls is None:
+            self._flags = ctypes.c_void_p(flags.data_ptr() if flags is not None else None)
+            self._sweep, self._run = self._lib.lbm_sweep, self._lib.lbm_run
+        else:
+            self._flags = ctypes.pointer(walls.native)
+            self._sweep, self._run = self._lib.lbm_sweep_walls, self._lib.lbm_run_walls
+            stream = torch.cuda.ExternalStream(stream_handle)
+            for t in walls.tensors:            # their memory outlives the sweeps queued on this stream
+                t.record_stream(stream)
 
     def sweep(self, src_ptr: int, dst_ptr: int, parity: int):
-        rc = self._lib.lbm_sweep(self.plan.handle, ctypes.c_void_p(src_ptr), ctypes.c_void_p(dst_ptr),
-                                 self._strides, self._flags, parity, None, self._stream)
+        rc = self._sweep(self.plan.handle, ctypes.c_void_p(src_ptr), ctypes.c_void_p(dst_ptr),
+                         self._strides, self._flags, parity, None, self._stream)
         if rc:
             N.check(rc, "lbm_sweep")
 
@@ -170,9 +180,9 @@ class BoundSweep:
     def run(self, a_ptr: int, b_ptr: int, first_parity: int, steps: int) -> bool:
         """`steps` sweeps in one call; returns True if a pull result ended in `b`."""
         in_b = ctypes.c_int(0)
-        N.check(self._lib.lbm_run(self.plan.handle, ctypes.c_void_p(a_ptr), ctypes.c_void_p(b_ptr),
-                                  self._strides, self._flags, first_parity, int(steps), ctypes.byref(in_b),
-                                  self._stream), "lbm_run")
+        N.check(self._run(self.plan.handle, ctypes.c_void_p(a_ptr), ctypes.c_void_p(b_ptr),
+                          self._strides, self._flags, first_parity, int(steps), ctypes.byref(in_b),
+                          self._stream), "lbm_run")
         return bool(in_b.value)
 
 
@@ -211,11 +221,11 @@ class LbKernel:
         return v
 
     def bind(self, pdfs: torch.Tensor, periodic, flags=None, ubb_velocities=None, params=None,
-             stream=None, fixed_density=None, ubb_options=None) -> BoundSweep:
+             stream=None, fixed_density=None, ubb_options=None, walls=None) -> BoundSweep:
         check_pdf_tensor(pdfs, self.q, self.update_rule.storage_dtype, "pdfs")
         dims = [s - 2 for s in pdfs.shape[:3]]
         plan = self.plan(dims, periodic, params or {}, ubb_velocities, fixed_density, ubb_options)
-        return BoundSweep(plan, pdfs.stride(), flags, _stream_handle(stream))
+        return BoundSweep(plan, pdfs.stride(), flags, _stream_handle(stream), walls)
 
     def _parity(self):
         ts = self.update_rule.timestep

@@ -221,7 +221,8 @@ class LatticeBoltzmannStep:
             k = self._kernels[0]
             flags = self._flags(k)
             self._bound_sweep = k.bind(self.pdfs, self.periodicity, flags, bh.ubb_velocities, self.kernel_params,
-                                       fixed_density=bh.fixed_density, ubb_options=bh.ubb_options)
+                                       fixed_density=bh.fixed_density, ubb_options=bh.ubb_options,
+                                       walls=bh.walls if flags is not None else None)
             if flags is not None:
                 bh.attach_links(self._bound_sweep.plan, self.pdfs, self._prev.idx if self._inplace else 0)
             self._bound_key = (id(bh._dev), bh._dev is None, tuple(sorted(self.kernel_params.items())),

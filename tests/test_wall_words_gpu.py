@@ -1,6 +1,5 @@
-"""Wall words (lbm_flags_finalize) against the flags themselves: a plan that did not finalize a flag
-field takes the walls of every cell from the flags, and both must give the same populations, bit for
-bit.  The box mixes NoSlip, two UBB numbers meeting in one cell, FixedDensity and per-link types
+"""Wall words (lbm_walls_build) against the flags themselves, with the finalizing plan's row summary and
+without: all must give the same populations, bit for bit.  The box mixes NoSlip, two UBB numbers meeting in one cell, FixedDensity and per-link types
 (bounced as NoSlip without link tables), on domain faces and around an obstacle, on sizes with
 remainders in every kernel's tiles."""
 import ctypes
@@ -49,19 +48,24 @@ def test_words_equal_flags(cuda, stencil, method, dtype, size, pattern, periodic
     stream = torch.cuda.current_stream().cuda_stream
     N.check(N.lib().lbm_flags_finalize(own.handle, ctypes.c_void_p(flags.data_ptr()), ctypes.c_void_p(stream)))
     q = kernel.method.stencil.Q
+    words = ctypes.c_int64(0)
+    N.check(N.lib().lbm_walls_size(own.handle, ctypes.byref(words)))
+    buffer, walls = torch.empty(words.value, dtype=torch.int32, device="cuda"), N.LbmWalls()
+    N.check(N.lib().lbm_walls_build(own.handle, ctypes.c_void_p(flags.data_ptr()), ctypes.c_void_p(buffer.data_ptr()),
+                                    ctypes.byref(walls), ctypes.c_void_p(stream)))
     gen = torch.Generator(device="cuda").manual_seed(5)
     results = []
     init = None
-    for plan in (own, other):
+    for plan, w in ((own, N.Walls(walls, (flags, buffer))), (own, None), (other, None)):
         a = create_pdf_array(size, q, dtype=dtype)
         b = a if pattern != "pull" else create_pdf_array(size, q, dtype=dtype)
         if init is None:
             init = (torch.rand(a.shape, generator=gen, device="cuda") - 0.5) * 1e-2
         a.copy_(init)
-        sweep = BoundSweep(plan, a.stride(), flags, stream)
+        sweep = BoundSweep(plan, a.stride(), flags, stream, w)
         in_b = sweep.run(a.data_ptr(), b.data_ptr(), 0, 5)
         results.append((b if in_b else a).clone())
     torch.cuda.synchronize()
-    assert torch.equal(results[0], results[1])
+    assert torch.equal(results[0], results[1]) and torch.equal(results[0], results[2])
     assert not torch.isnan(results[0].float()).any()
     assert (results[0].float() - init.to(results[0].dtype).float()).abs().max() > 1e-4
