@@ -296,6 +296,7 @@ typedef struct LbmBatchTiling {
 /* Validates every domain (bounds inside buffers of buffer_elems elements and a flag buffer of
  * flags_bytes bytes, no two domains overlapping), marks the near-wall cells of every domain's
  * flags in place (as lbm_flags_finalize), uploads the per-domain arguments and the tile table.
+ * The walls are taken from the flags here, once: flags that change later need a new batch.
  * In-place patterns take buffer_b == NULL or buffer_a.  The buffers stay owned by the caller. */
 int lbm_batch_create(const LbmPlanDesc* common, const LbmDomainDesc* domains, int n_domains, void* buffer_a,
                      void* buffer_b, int64_t buffer_elems, uint8_t* flags, int64_t flags_bytes,

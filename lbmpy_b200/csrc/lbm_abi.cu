@@ -1537,10 +1537,13 @@ int lbm_batch_create(const LbmPlanDesc* common, const LbmDomainDesc* domains, in
     size_t wall_words = 0;
     for (int k = 0; k < n_domains; ++k)
         if (domains[k].flags_offset >= 0) wall_words += size_t(args[k].g.nx) * args[k].g.ny * args[k].g.nz;
-    if (wall_words > 0) e = cudaMalloc(&b->d_walls, sizeof(uint32_t) * wall_words);
+    if (wall_words > 0 && cudaMalloc(&b->d_walls, sizeof(uint32_t) * wall_words) != cudaSuccess) {
+        b->d_walls = nullptr;          // without the memory the sweeps take the walls from the flags
+        cudaGetLastError();
+    }
     wall_words = 0;
-    for (int k = 0; k < n_domains && e == cudaSuccess; ++k) {
-        if (domains[k].flags_offset < 0) continue;
+    for (int k = 0; k < n_domains; ++k) {
+        if (domains[k].flags_offset < 0 || b->d_walls == nullptr) continue;
         args[k].g.walls = args[n_domains + k].g.walls = b->d_walls + wall_words;
         wall_words += size_t(args[k].g.nx) * args[k].g.ny * args[k].g.nz;
     }
@@ -1558,7 +1561,7 @@ int lbm_batch_create(const LbmPlanDesc* common, const LbmDomainDesc* domains, in
         if (q == 19) k_flags_finalize<19><<<grid, block>>>(g);
         else k_flags_finalize<27><<<grid, block>>>(g);
         e = cudaGetLastError();
-        if (e == cudaSuccess) e = launch_wall_words(q, g, const_cast<uint32_t*>(g.walls), nullptr);
+        if (e == cudaSuccess && g.walls != nullptr) e = launch_wall_words(q, g, const_cast<uint32_t*>(g.walls), nullptr);
     }
     if (e == cudaSuccess) e = cudaDeviceSynchronize();
     if (e != cudaSuccess) {
