@@ -17,8 +17,11 @@ using MacroLauncher = cudaError_t (*)(const MacroArgs&, dim3, dim3, cudaStream_t
 template <class S, class R, int Q, int MK, int PAT>
 cudaError_t launch_sweep(const SweepArgs& a, dim3 grid, dim3 block, cudaStream_t s) {
     // SRT/TRT pull with FP32 storage runs at memory speed; without the wall code its 48 registers hold the
-    // loads in the better order (D3Q19 512^3: 3.20 ms, with it 3.26 ms).
-    if constexpr (MK == MK_POP && PAT == PAT_PULL && std::is_same<S, float>::value)
+    // loads in the better order (D3Q19 512^3: 3.20 ms, with it 3.26 ms).  The general MRT and cumulant
+    // transforms leave few registers for it (256x128x128 periodic: D3Q19 MRT pull FP32 128.0 -> 126.4 us; FP64
+    // D3Q27 MRT pull 470 -> 446, cumulant with general rates push 482 -> 462, AA 505 -> 479 us).
+    if constexpr (((MK == MK_POP || (MK == MK_MRT && Q == 19)) && PAT == PAT_PULL && std::is_same<S, float>::value) ||
+                  (Q == 27 && (MK == MK_MRT || MK == MK_CUM) && std::is_same<S, double>::value))
         if (a.g.flags == nullptr) return launch_chained(&k_sweep<S, R, Q, MK, PAT, false>, grid, block, 0, s, a);
     return launch_chained(&k_sweep<S, R, Q, MK, PAT>, grid, block, 0, s, a);
 }
@@ -31,6 +34,10 @@ cudaError_t launch_set_eq(const MacroArgs& a, dim3 grid, dim3 block, cudaStream_
 
 template <class S, int Q, int MK, int PAT>
 cudaError_t launch_sweep_pair(const SweepArgs& a, dim3 grid, dim3 block, cudaStream_t s) {
+    // The general MRT transform of two cells spills with the wall code beside it (D3Q19 FP16 pull 256x128x128
+    // periodic: 164 us, without it 124 us).
+    if constexpr (MK == MK_MRT)
+        if (a.g.flags == nullptr) return launch_chained(&k_sweep_pair<S, Q, MK, PAT, false>, grid, block, 0, s, a);
     return launch_chained(&k_sweep_pair<S, Q, MK, PAT>, grid, block, 0, s, a);
 }
 

@@ -105,19 +105,25 @@ template <class S> __device__ __forceinline__ S* at(S* field, unsigned slot_off,
 // How a sweep addresses the slots of a field.
 //   ADDR_INDEX    one 32-bit element index per access: the least work ahead of the first load, for the
 //                 SRT/TRT sweeps, which run at memory speed (D3Q19 TRT pull FP32 256^3: 402 us, with
-//                 uniform addresses 406 us)
+//                 uniform addresses 406 us), and for the general MRT and cumulant transforms, which have no
+//                 registers left for the shared parts (256x128x128, uniform -> index: D3Q27 MRT FP32 pull
+//                 227 -> 205 us, D3Q19 MRT FP32 AA 155 -> 150, cumulant with general rates FP32 pull (two cells
+//                 a thread) 261 -> 245, FP64 EsoTwist channel 527 -> 510)
 //   ADDR_UNIFORM  slot part uniform, cell part shared by the slots of one offset (at()): fewer
 //                 instructions, for the methods limited by their number (D3Q27 cumulant AA FP32
-//                 256x128x128: 164.6 -> 157.8 us, D3Q19 MRT pull FP32 256^3: 521 -> 493 us, both with
-//                 the FP32 copies of the physics)
+//                 256x128x128: 164.6 -> 157.8 us, both with the FP32 copies of the physics), among them the
+//                 D3Q19 MRT pull sweep (FP32 256x128x128: 128.3 us with indices, 125.7 so)
 //   ADDR_WALK     strides read from shared memory (batched sweep) are ordinary registers, where the
 //                 compiler keeps the products of all slots from the loads to the stores and spills:
 //                 the slot address is walked, hidden from it step by step (D3Q19 MRT batch at 80
-//                 registers: 48 -> 40 bytes of stack, SRT/TRT none)
+//                 registers: 48 -> 40 bytes of stack).
 __device__ __forceinline__ unsigned eidx(unsigned slot_off, int cell_off) { return slot_off + unsigned(cell_off); }
 
 enum : int { ADDR_INDEX = 0, ADDR_UNIFORM = 1, ADDR_WALK = 2 };
-template <int MK> struct AddrOf { static constexpr int value = MK == MK_POP ? ADDR_INDEX : ADDR_UNIFORM; };
+template <int Q, int MK, int PAT> struct AddrOf {
+    static constexpr bool index = MK == MK_POP || MK == MK_CUM || (MK == MK_MRT && !(Q == 19 && PAT == PAT_PULL));
+    static constexpr int value = index ? ADDR_INDEX : ADDR_UNIFORM;
+};
 
 template <int ADDR, class S> __device__ __forceinline__ S* addr(S* field, unsigned slot_off, int cell_off) {
     if constexpr (ADDR == ADDR_INDEX) return field + eidx(slot_off, cell_off);
@@ -274,7 +280,7 @@ __device__ __forceinline__ void bounce_back(R (&f)[Q], const SweepArgs& a, const
 
 // The whole update of one cell: pull through the accessor, fused bounce-back, collision, push
 // through the accessor.  Shared by the single-domain and the batched sweeps.
-template <class S, class R, int Q, int MK, int PAT, int ADDR = AddrOf<MK>::value, bool WALLS = true>
+template <class S, class R, int Q, int MK, int PAT, int ADDR = AddrOf<Q, MK, PAT>::value, bool WALLS = true>
 __device__ __forceinline__ void sweep_cell(const SweepArgs& a, int x, int y, int z) {
     using A = Access<PAT>;
     const Grid& g = a.g;
@@ -355,6 +361,15 @@ template <> struct SweepMinBlocks<float, 27, MK_POP, PAT_AA_ODD> { static conste
 template <> struct SweepMinBlocks<float, 27, MK_POP, PAT_AA_EVEN> { static constexpr int value = 3; };
 template <> struct SweepMinBlocks<float, 19, MK_MRT, PAT_PULL> { static constexpr int value = 4; };
 template <> struct SweepMinBlocks<float, 27, MK_MRT, PAT_PULL> { static constexpr int value = 3; };
+// These took registers for a block less, left alone, with uniform addresses (256x128x128: D3Q27 MRT FP32 AA 154
+// and 168, 345 us, now 107 and 128, 235 us; D3Q19 MRT AA even FP32 95, 159 -> 138 us; FP16 and BF16 116 and 108,
+// now 80; cumulant push FP64 147, 394 us, now 112, 285 us).  At most 12 bytes spill.
+template <> struct SweepMinBlocks<float, 27, MK_MRT, PAT_AA_EVEN> { static constexpr int value = 2; };
+template <> struct SweepMinBlocks<float, 27, MK_MRT, PAT_AA_ODD> { static constexpr int value = 2; };
+template <> struct SweepMinBlocks<float, 19, MK_MRT, PAT_AA_EVEN> { static constexpr int value = 3; };
+template <> struct SweepMinBlocks<__half, 19, MK_MRT, PAT_AA_EVEN> { static constexpr int value = 3; };
+template <> struct SweepMinBlocks<__nv_bfloat16, 19, MK_MRT, PAT_AA_EVEN> { static constexpr int value = 3; };
+template <> struct SweepMinBlocks<double, 27, MK_CUM1, PAT_PUSH> { static constexpr int value = 2; };
 
 // WALLS false: for domains without flags.
 template <class S, class R, int Q, int MK, int PAT, bool WALLS = true>
@@ -364,7 +379,7 @@ __global__ void __launch_bounds__(256, SweepMinBlocks<S, Q, MK, PAT>::value) k_s
     const int y = blockIdx.y * blockDim.y + threadIdx.y;
     const int z = blockIdx.z;
     if (x >= a.g.nx || y >= a.g.ny) return;
-    sweep_cell<S, R, Q, MK, PAT, AddrOf<MK>::value, WALLS>(a, x, y, z);
+    sweep_cell<S, R, Q, MK, PAT, AddrOf<Q, MK, PAT>::value, WALLS>(a, x, y, z);
 }
 
 // Pipelined z-columns: each thread sweeps a.zc consecutive cells along z and issues the loads of
@@ -410,7 +425,7 @@ __global__ void __launch_bounds__(256, 2) k_sweep_zpipe(const SweepArgs a) {
         NbrOffsets nb;
         nb.init(g, x, y, z);
         const int cell = (x + 1) + (y + 1) * g.sy + (z + 1) * g.sz;
-        if (w != 0) bounce_back<S, R, Q, PAT, AddrOf<MK>::value>(f, a, nb, cell, x, y, z, w);
+        if (w != 0) bounce_back<S, R, Q, PAT, AddrOf<Q, MK, PAT>::value>(f, a, nb, cell, x, y, z, w);
         collide<R, Q, MK>(f, a.p);
 #pragma unroll
         for (int i = 0; i < Q; ++i) {

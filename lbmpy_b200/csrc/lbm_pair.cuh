@@ -101,13 +101,14 @@ template <> struct PairMinBlocks<__half> { static constexpr int value = 6; };
 template <> struct PairMinBlocks<__nv_bfloat16> { static constexpr int value = 6; };
 template <> struct PairMinBlocks<e3m12> { static constexpr int value = 6; };
 
-template <class S, int Q, int MK, int PAT>
+// WALLS false: for domains without flags.
+template <class S, int Q, int MK, int PAT, bool WALLS = true>
 __global__ void __launch_bounds__(32 * PAIR_ROWS, PairMinBlocks<S>::value) k_sweep_pair(const SweepArgs a) {
     static_assert(PAT == PAT_PULL || PAT == PAT_AA_EVEN || PAT == PAT_AA_ODD, "pair sweep: pull and AA");
     using L = Lat<Q>;
     using A = Access<PAT>;
     using PS = Pair<S>;
-    constexpr int ADDR = AddrOf<MK>::value;
+    constexpr int ADDR = AddrOf<Q, MK, PAT>::value;
     chain_wait();
     const Grid& g = a.g;
     const int lane = threadIdx.x;
@@ -131,7 +132,7 @@ __global__ void __launch_bounds__(32 * PAIR_ROWS, PairMinBlocks<S>::value) k_swe
     // The wall words come before the populations here: with the row's answer looked at after them (as
     // the one-cell sweep does) the loads no longer overlap the lane exchanges (D3Q27 cumulant pull FP32
     // 256x128x128 152 -> 184 us, D3Q19 TRT pull FP16 256^3 276 -> 293 us).
-    const uint32_t wA = wall_word<Q>(g, x0, y, z), wB = wall_word<Q>(g, x0 + 1, y, z);
+    const uint32_t wA = WALLS ? wall_word<Q>(g, x0, y, z) : 0u, wB = WALLS ? wall_word<Q>(g, x0 + 1, y, z) : 0u;
 
     F2 f[Q];
 #pragma unroll

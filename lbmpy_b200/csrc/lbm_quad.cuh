@@ -63,7 +63,7 @@ __global__ void __launch_bounds__(32 * QUAD_ROWS, 4) k_sweep_quad(const SweepArg
     static_assert(PAT == PAT_PULL || PAT == PAT_AA_EVEN || PAT == PAT_AA_ODD, "quad sweep: pull and AA");
     using L = Lat<Q>;
     using A = Access<PAT>;
-    constexpr int ADDR = AddrOf<MK>::value;
+    constexpr int ADDR = AddrOf<Q, MK, PAT>::value;
     chain_wait();
     const Grid& g = a.g;
     const int lane = threadIdx.x;

@@ -269,7 +269,7 @@ __global__ void __launch_bounds__(W) k_sweep_staged(const SweepArgs a, const int
             NbrOffsets nb;
             nb.init(g, x, t.y, t.z);
             const int cell = (x + 1) + (t.y + 1) * g.sy + (t.z + 1) * g.sz;
-            if (w != 0) bounce_back<S, R, Q, PAT, AddrOf<MK>::value>(f, a, nb, cell, x, t.y, t.z, w);
+            if (w != 0) bounce_back<S, R, Q, PAT, AddrOf<Q, MK, PAT>::value>(f, a, nb, cell, x, t.y, t.z, w);
             const R om = collide<R, Q, MK>(f, a.p);
 #pragma unroll
             for (int i = 0; i < Q; ++i) {

@@ -11,6 +11,7 @@ import lbmpy_b200 as L
 from lbmpy_b200 import _native as N
 from lbmpy_b200.fields import create_flag_array, create_pdf_array
 from lbmpy_b200.kernel import BoundSweep, build_desc
+from tests.test_gpu_parity import FP64_TOL, _interior, make_pair, pop_rel_linf, run_pair
 
 pytestmark = pytest.mark.gpu
 
@@ -77,6 +78,35 @@ def test_sweeps_without_wall_code(cuda, stencil, method, dtype, pattern, size):
     eps = {"float32": 2e-7, "float16": 2 ** -10, "bfloat16": 2 ** -7}[dtype]
     scale = want.double().norm()
     assert (got.double() - want.double()).norm() <= 4 * eps * scale
+
+
+@pytest.mark.parametrize("stencil,dtype,pattern", [("D3Q19", "float32", "pull"), ("D3Q19", "float16", "pull"),
+                                                   ("D3Q19", "bfloat16", "aa"), ("D3Q27", "float32", "aa")])
+@pytest.mark.parametrize("size", [(2, 3, 2), (34, 6, 3), (130, 5, 3)])
+@pytest.mark.parametrize("force", [None, (1e-4, -2e-5, 3e-5)], ids=["plain", "force"])
+def test_general_mrt_pairs_without_wall_code(cuda, stencil, dtype, pattern, size, force, monkeypatch):
+    monkeypatch.setenv("LBM_B200_PAIR", "1")
+    rates = [1.8, 1.6, 1.1, 1.2] + ([1.3, 1.1] if stencil == "D3Q27" else [])
+    got, name = _sweep(size, 4, stencil, "mrt", dtype, pattern, rates, force=force)
+    want, same = _sweep(size, 4, stencil, "mrt", dtype, pattern, rates, flags=True, force=force)
+    assert name == same == "pair"
+    # the same operations up to contraction, rounded to storage four times
+    eps = {"float32": 2e-7, "float16": 2 ** -10, "bfloat16": 2 ** -7}[dtype]
+    assert (got.double() - want.double()).norm() <= 4 * eps * want.double().norm()
+
+
+@pytest.mark.parametrize("method,pattern,dtype", [("mrt", "pull", "float64"), ("mrt", "aa", "float64"),
+                                                  ("cumulant", "pull", "float64"), ("cumulant", "aa", "float64"),
+                                                  ("cumulant", "push", "float64"), ("cumulant", "esotwist", "float64")])
+@pytest.mark.parametrize("size", [(2, 3, 2), (34, 6, 3), (130, 5, 3)])
+def test_general_transforms_without_wall_code_match_oracle(cuda, method, pattern, dtype, size):
+    rates = [1.8, 1.6, 1.1, 1.2, 1.3, 1.1] if method == "mrt" else [1.8, 1.0] + [1.1] * 8
+    step, orc, f, flags, ubb, prev = make_pair("D3Q27", method, size, pattern, dtype, relaxation_rates=rates,
+                                               compressible=True)
+    res, _ = run_pair(step, orc, f, flags, ubb, prev, 20, pattern, (1, 1, 1))
+    assert flags is None and step.sweep_variant() == "cell"
+    err = pop_rel_linf(_interior(step.pdfs), res[1:-1, 1:-1, 1:-1], step.method.weights)
+    assert err < FP64_TOL
 
 
 @pytest.mark.parametrize("stencil,higher", [("D3Q19", 2), ("D3Q27", 4)])
