@@ -116,7 +116,8 @@ template <class S> __device__ __forceinline__ S* at(S* field, unsigned slot_off,
 //   ADDR_WALK     strides read from shared memory (batched sweep) are ordinary registers, where the
 //                 compiler keeps the products of all slots from the loads to the stores and spills:
 //                 the slot address is walked, hidden from it step by step (D3Q19 MRT batch at 80
-//                 registers: 48 -> 40 bytes of stack).
+//                 registers: 48 -> 40 bytes of stack).  Where the collision spills anyway the walk can cost
+//                 more than it saves (AddrOfBatch)
 __device__ __forceinline__ unsigned eidx(unsigned slot_off, int cell_off) { return slot_off + unsigned(cell_off); }
 
 enum : int { ADDR_INDEX = 0, ADDR_UNIFORM = 1, ADDR_WALK = 2 };
@@ -483,8 +484,21 @@ struct BatchArgs {
     int parity;                   // selects which half of `domains` (src/dst swapped) to use
 };
 
-// Resident 256-thread blocks per SM that the batched sweep is compiled for.
-template <class S, int Q, int MK> struct BatchMinBlocks { static constexpr int value = 3; };
+// How the batched sweep addresses the slots of its domains' fields: indices where the walk measured slower (32
+// domains of 32^3 to 96^3, walk -> index: D3Q19 MRT FP64 pull 876 -> 768 us a sweep, D3Q27 FP32 AA SRT/TRT
+// 577 -> 543, MRT 915 -> 859, central moments without walls 586 -> 566; the cumulant FP64 pull 926 -> 950 and
+// FP32 pull 552 -> 576 walk).
+template <class S, int Q, int MK, int PAT> struct AddrOfBatch {
+    static constexpr bool f64 = std::is_same<S, double>::value;
+    static constexpr bool index = MK == MK_CM || (f64 && MK == MK_MRT) ||
+                                  (!f64 && PAT != PAT_PULL && (MK == MK_CUM || (Q == 27 && (MK == MK_MRT || MK == MK_POP))));
+    static constexpr int value = index ? ADDR_INDEX : ADDR_WALK;
+};
+
+// Resident 256-thread blocks per SM that the batched sweep is compiled for.  FP64 spills 300 to 1300 bytes at 3
+// (80 registers), 0 to 160 at 2 (the same domains, 3 -> 2: D3Q27 cumulant AA 1177 -> 896 us a sweep, TRT pull
+// 1072 -> 830, D3Q19 MRT pull 1142 -> 768; without walls 1035 -> 759, 946 -> 721, 1097 -> 659).
+template <class S, int Q, int MK> struct BatchMinBlocks { static constexpr int value = std::is_same<S, double>::value ? 2 : 3; };
 
 template <class S, class R, int Q, int MK, int PAT>
 __global__ void __launch_bounds__(256, BatchMinBlocks<S, Q, MK>::value) k_sweep_batched(const BatchArgs b) {
@@ -511,7 +525,7 @@ __global__ void __launch_bounds__(256, BatchMinBlocks<S, Q, MK>::value) k_sweep_
         if (x < sa.g.nx && y < sa.g.ny) {
             const int z1 = min(tile.z0 + b.cells_z, sa.g.nz);
 #pragma unroll 1
-            for (int z = tile.z0; z < z1; ++z) sweep_cell<S, R, Q, MK, PAT, ADDR_WALK>(sa, x, y, z);
+            for (int z = tile.z0; z < z1; ++z) sweep_cell<S, R, Q, MK, PAT, AddrOfBatch<S, Q, MK, PAT>::value>(sa, x, y, z);
         }
     }
 }

@@ -20,5 +20,6 @@ template <int PAT> struct SweepMinBlocks<double, 19, MK_MRT1, PAT> { static cons
 template <int PAT> struct SweepMinBlocks<float, 27, MK_MRT1, PAT> { static constexpr int value = 3; };
 template <int PAT> struct SweepMinBlocks<double, 27, MK_MRT1, PAT> { static constexpr int value = 2; };
 template <> struct BatchMinBlocks<float, 19, MK_MRT1> { static constexpr int value = 4; };
+template <int Q> struct BatchMinBlocks<double, Q, MK_MRT1> { static constexpr int value = 3; };
 
 }  // namespace lbm
