@@ -226,7 +226,9 @@ SweepLauncher quad_launcher(const LbmPlan* p, int pat) {
 // nx a multiple of 4 and interior cell x = 0 of every row and slot on an 8-byte boundary.
 // Default policy, from B200 measurements: SRT/TRT (D3Q19 TRT FP16 pull 61.3 -> 68.2 GLUPS at
 // 256^3, 62.8 -> 70.0 at 512^3); not the moment-space methods, whose larger collision state
-// spills (MRT) or loses occupancy (cumulant AA: 29.0 -> 25.9).
+// spills (MRT) or loses occupancy (cumulant AA: 29.0 -> 25.9).  The MRT form for higher moments relaxed by 1
+// does neither; of its D3Q19 sweeps at 256x128x128 FP16 AA gains over the pair sweep (74.8 -> 70.3 us,
+// channel 83.7 -> 77.8), FP16 pull does not (64.2 -> 64.3), e3m12 pull loses (93.5 -> 97.5): opt-in as well.
 bool quad_applicable(const LbmPlan* p, const void* src, const void* dst, const int64_t s[4], int pat,
                      const float* omega_out) {
     if (p->use_quad == 0 || (p->use_quad < 0 && p->mk != MK_POP)) return false;

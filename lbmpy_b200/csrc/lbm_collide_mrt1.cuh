@@ -27,8 +27,8 @@ template <int Q, class R> constexpr double mrt1_odd(int c2) {
 // (mrt1_odd), which leaves rounding noise alone, as a collision that adds small changes does.
 //
 // Ten sums of the populations are all that is kept of them: about half the arithmetic of the
-// transforms of collide_mrt and fewer registers (D3Q19 FP32 pull: 48 registers without spilling, collide_mrt 64
-// with).
+// transforms of collide_mrt and fewer registers (D3Q19 FP32 pull: 48 registers with 12 bytes spilled, collide_mrt 64 with
+// 20).
 template <int Q, class R, class P>
 __device__ __forceinline__ R collide_mrt1(R (&f)[Q], const P& p) {
     using L = Lat<Q>;

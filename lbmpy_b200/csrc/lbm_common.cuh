@@ -12,8 +12,8 @@ namespace lbm {
 
 enum StoreType : int { ST_F64 = 0, ST_F32 = 1, ST_F16 = 2, ST_BF16 = 3, ST_E3M12 = 4 };
 // SRT/TRT | raw-moment MRT | cumulant | cumulant with every order >= 3 relaxed by 1 | with a learned
-// closure | D3Q27 central moments
-enum MethodKind : int { MK_POP = 0, MK_MRT = 1, MK_CUM = 2, MK_CUM1 = 3, MK_CUM1_MLP = 4, MK_CM = 5 };
+// closure | D3Q27 central moments | raw-moment MRT with every moment of order >= 3 relaxed by 1
+enum MethodKind : int { MK_POP = 0, MK_MRT = 1, MK_CUM = 2, MK_CUM1 = 3, MK_CUM1_MLP = 4, MK_CM = 5, MK_MRT1 = 6 };
 enum PatternKind : int {
     PAT_PULL = 0, PAT_AA_EVEN = 1, PAT_AA_ODD = 2, PAT_ESO_EVEN = 3, PAT_ESO_ODD = 4,
     PAT_PUSH = 5, PAT_EPULL_EVEN = 6, PAT_EPULL_ODD = 7, PAT_EPUSH_EVEN = 8, PAT_EPUSH_ODD = 9

@@ -188,8 +188,8 @@ __device__ __forceinline__ R load_f_out(const SweepArgs& a, int x, int y, int z,
 // in-place sweep those cells update concurrently, so k_boundary_prepass stores those links' values
 // where the sweep reads them before the sweep runs, as lbmpy's boundary kernel does.
 //
-// Bound by latency: a warp with one such cell waits for every load here, and with walls at the row
-// ends every warp of a cavity has one.  The directions come as one word per cell (`w`, wall_word), so
+// Bound by latency: a warp with one such cell waits for every load here, and in a cavity the warps at
+// the row ends and all of the rows along the other walls have one.  The directions come as one word per cell (`w`, wall_word), so
 // the bounced populations are fetched together after a single load, where a flag per neighbour cost
 // up to Q - 1 dependent round trips, one after another.
 template <class S, class R, int Q, int PAT, int ADDR>
@@ -348,8 +348,9 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs& a, int x, int y, int
 // of the copy bandwidth; 0.92 at 64).  These hot variants are held to register counts checked
 // for spills with -Xptxas -v: 128 (2 blocks), 80 (3), 64 (4) and 48 (5).  The cumulant's three take 64
 // without spilling (odd: 80 before the FP32 copies of the physics and uniform addresses; pull: 90, 192 us
-// for 256x128x128, 155 us at 64).  D3Q27 SRT/TRT AA takes 80 in both parities: at 64 both spill (force-driven AA
-// channel 256x128x128 213 us a sweep, 188 us at 80; without the force 184 us with the even one at 64, 173 us).
+// for 256x128x128, 155 us at 64).  D3Q27 SRT/TRT AA takes 80 in both parities, where the odd one spills 48 bytes:
+// at 64 both spill more (force-driven AA channel 256x128x128 213 us a sweep, 188 us at 80; without the force
+// 184 us with the even one at 64, 173 us).
 template <class S, int Q, int MK, int PAT> struct SweepMinBlocks { static constexpr int value = 1; };
 template <> struct SweepMinBlocks<float, 27, MK_CUM1, PAT_AA_ODD> { static constexpr int value = 4; };
 template <> struct SweepMinBlocks<double, 19, MK_POP, PAT_PULL> { static constexpr int value = 2; };

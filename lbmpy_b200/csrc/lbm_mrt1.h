@@ -5,8 +5,6 @@
 
 namespace lbm {
 
-constexpr int MK_MRT1 = 6;
-
 SweepLauncher sweep_q19_mrt1(int store, int pat);
 SweepLauncher sweep_pair_q19_mrt1(int store, int pat);
 SweepLauncher sweep_quad_q19_mrt1(int store, int pat);
