@@ -177,17 +177,18 @@ def i64_array(values):
 
 
 class Walls:
-    """An LbmWalls and the tensors whose device memory it points to."""
+    """An LbmWalls, the tensors whose device memory it points to and the stream they were allocated on."""
 
-    def __init__(self, native: LbmWalls, tensors):
+    def __init__(self, native: LbmWalls, tensors, stream: int):
         self.native = native
         self.tensors = tuple(tensors)
+        self.stream = stream
 
     def slab(self, z0: int, nz: int) -> "Walls":
         """The walls of interior planes [z0, z0 + nz)."""
         out = LbmWalls()
         check(lib().lbm_walls_slab(ctypes.byref(self.native), int(z0), int(nz), ctypes.byref(out)), "lbm_walls_slab")
-        return Walls(out, self.tensors)
+        return Walls(out, self.tensors, self.stream)
 
 
 class Plan:

@@ -613,8 +613,8 @@ class LatticeBoltzmannBoundaryHandling:
         key = (int(plan.desc.stencil), tuple(plan.desc.periodic))
         if self._dev is None or self._finalized_for != key:
             t = torch.from_numpy(self._host.copy()).to(self.device).permute(2, 1, 0)
-            stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
-            N.check(N.lib().lbm_flags_finalize(plan.handle, ctypes.c_void_p(t.data_ptr()), stream),
+            stream = torch.cuda.current_stream().cuda_stream
+            N.check(N.lib().lbm_flags_finalize(plan.handle, ctypes.c_void_p(t.data_ptr()), ctypes.c_void_p(stream)),
                     "lbm_flags_finalize")
             self._walls = self._build_walls(plan, t, stream)
             self._dev = t
@@ -634,8 +634,9 @@ class LatticeBoltzmannBoundaryHandling:
             return None
         w = N.LbmWalls()
         N.check(N.lib().lbm_walls_build(plan.handle, ctypes.c_void_p(flags.data_ptr()),
-                                        ctypes.c_void_p(buffer.data_ptr()), ctypes.byref(w), stream), "lbm_walls_build")
-        return N.Walls(w, (flags, buffer))
+                                        ctypes.c_void_p(buffer.data_ptr()), ctypes.byref(w),
+                                        ctypes.c_void_p(stream)), "lbm_walls_build")
+        return N.Walls(w, (flags, buffer), stream)
 
     @property
     def walls(self) -> Optional[N.Walls]:

@@ -159,9 +159,10 @@ class BoundSweep:
         else:
             self._flags = ctypes.pointer(walls.native)
             self._sweep, self._run = self._lib.lbm_sweep_walls, self._lib.lbm_run_walls
-            stream = torch.cuda.ExternalStream(stream_handle)
-            for t in walls.tensors:            # their memory outlives the sweeps queued on this stream
-                t.record_stream(stream)
+            if stream_handle != walls.stream:      # their memory outlives the sweeps queued on this stream too
+                stream = torch.cuda.ExternalStream(stream_handle)
+                for t in walls.tensors:
+                    t.record_stream(stream)
 
     def sweep(self, src_ptr: int, dst_ptr: int, parity: int):
         rc = self._sweep(self.plan.handle, ctypes.c_void_p(src_ptr), ctypes.c_void_p(dst_ptr),

@@ -1,5 +1,6 @@
 """Wall words (lbm_walls_build) against the flags themselves, with the finalizing plan's row summary and
-without: all must give the same populations, bit for bit.  The box mixes NoSlip, two UBB numbers meeting in one cell, FixedDensity and per-link types
+without: all must give the same populations, bit for bit.  The box mixes NoSlip, two UBB numbers meeting
+in one cell, FixedDensity and per-link types
 (bounced as NoSlip without link tables), on domain faces and around an obstacle, on sizes with
 remainders in every kernel's tiles."""
 import ctypes
@@ -56,7 +57,7 @@ def test_words_equal_flags(cuda, stencil, method, dtype, size, pattern, periodic
     gen = torch.Generator(device="cuda").manual_seed(5)
     results = []
     init = None
-    for plan, w in ((own, N.Walls(walls, (flags, buffer))), (own, None), (other, None)):
+    for plan, w in ((own, N.Walls(walls, (flags, buffer), stream)), (own, None), (other, None)):
         a = create_pdf_array(size, q, dtype=dtype)
         b = a if pattern != "pull" else create_pdf_array(size, q, dtype=dtype)
         if init is None:

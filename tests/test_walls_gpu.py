@@ -109,3 +109,24 @@ def test_without_the_memory_the_sweeps_use_the_flags(cuda, monkeypatch):
     assert step.boundary_handling.walls is None
     torch.cuda.synchronize()
     assert torch.equal(step.pdfs, want.pdfs)
+
+
+def test_walls_given_back_while_another_stream_still_sweeps(cuda):
+    """New boundaries drop the walls of the old ones; their memory must not be handed out again while sweeps
+    queued on another stream than the one they were built on still read them."""
+    want = _step(obstacle=BOX)
+    want.run_sweeps(40)
+    step = _step(obstacle=BOX)
+    step._bound()                                   # built on the current stream
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        step.run_sweeps(40)
+        got = step.pdfs
+        step.boundary_handling.set_boundary(L.NoSlip(), L.slice_from_direction("N", 3))
+        step._bound()                               # lets go of the first walls
+    n = int(np.prod(SIZE)) + 2 * SIZE[2]
+    junk = [torch.full((n,), -1, dtype=torch.int32, device="cuda") for _ in range(8)]
+    torch.cuda.synchronize()
+    assert torch.equal(got, want.pdfs)
+    del junk
